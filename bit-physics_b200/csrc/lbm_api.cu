@@ -1,6 +1,7 @@
 // lbm_api.cu -- the C ABI of include/lbm_d3q19.h: lattice handles, state
 // transfer, the step loop and the stateless reference functions.
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -83,6 +84,23 @@ void fill_constants(Params& P)
     for (int i = 7; i < Q; ++i) P.w[i] = one / thirtysix;
 }
 
+// 1 / y as an unevaluated sum for div_exact: hi = RN(1 / y); 1 - y hi is exact
+// in one fma, lo is the rest of the reciprocal rounded.
+void split_reciprocal(double y, double* hi, double* lo)
+{
+    *hi = 1.0 / y;
+    *lo = std::fma(-y, *hi, 1.0) / y;
+}
+
+// The constants that depend on tau alone.
+void set_tau_constants(Params& P, double tau)
+{
+    P.tau = tau;
+    split_reciprocal(tau, &P.tau_rhi, &P.tau_rlo);
+    P.pref64 = 1.0 - 0.5 / tau;
+    P.tau_fast = tau >= 0.0625 && tau <= 1048576.0;
+}
+
 void init_geometry(Params& P, int nx, int ny, int nz)
 {
     std::memset(&P, 0, sizeof(P));
@@ -98,7 +116,8 @@ void init_geometry(Params& P, int nx, int ny, int nz)
     P.periodic = 7;
     P.wall_sum_pairwise = (long long)nx * nz == 1;
     fill_constants(P);
-    P.tau = 1.0;
+    split_reciprocal(P.cs2, &P.cs2_rhi, &P.cs2_rlo);
+    set_tau_constants(P, 1.0);
 }
 
 bool dims_ok(long long nx, long long ny, long long nz)
@@ -127,7 +146,7 @@ void rebuild_params(lbm_lattice* h)
     P.err = h->err;
     P.force = h->force;
     P.porosity = h->poro;
-    P.tau = d.tau;
+    set_tau_constants(P, d.tau);
     for (int f = 0; f < 6; ++f)
         for (int a = 0; a < 3; ++a) {
             P.wall_u[f][a] = d.wall_velocity[f][a];
@@ -1337,7 +1356,7 @@ int lbm_bgk_step_dev(const double* f, double* f_out, double tau, const double* f
     if (rc) return rc;
     if (!f || !f_out || f == f_out) return fail(LBM_ERR_INVALID, "null or aliased pointer");
     if ((rc = check_dev_ptrs({{f, "f"}, {force, "force"}, {f_out, "f_out"}}))) return rc;
-    P.tau = tau;
+    set_tau_constants(P, tau);
     return finish(ref_bgk_step(P, f, force, f_out, (cudaStream_t)stream), "bgk_step", (cudaStream_t)stream);
 }
 

@@ -474,7 +474,7 @@ __global__ void k_ref_stream(Params P, const double* __restrict__ fin, double* _
 // collide-in-place + push to (x + c_d) mod n.  Each output element is written
 // by exactly one thread.
 template <int FM>
-__global__ void k_ref_bgk_step(Params P, const double* __restrict__ f, double* __restrict__ fout)
+__global__ void k_ref_bgk_step(const __grid_constant__ Params P, const double* __restrict__ f, double* __restrict__ fout)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.n) return;

@@ -181,7 +181,7 @@ __device__ __forceinline__ void step_single(const Params& P, const Streams<typen
 // 2 blocks): 17.1 against 14.5 GLUPS on the 256x128x128 sphere channel with
 // 128-thread blocks; f64 results do not depend on it (no contraction).
 template <class M, int FM, int OUT>
-__global__ void __launch_bounds__(256, 3) k_step(Params P, Streams<typename M::T> S, Outputs<typename M::C> out)
+__global__ void __launch_bounds__(256, 3) k_step(const __grid_constant__ Params P, Streams<typename M::T> S, Outputs<typename M::C> out)
 {
     if constexpr ((OUT & OUT_SUMS) != 0) reduce_prev(out);
     const int t = P.cell0 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -828,7 +828,7 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* b, int* err, unsigned exp
 // that runs out (expected arrivals that never come) raises *P.err, and every
 // block leaves at its next barrier.
 template <class M, int FM, int VEC>
-__global__ void __launch_bounds__(256) k_step_persistent(Params P, Streams<typename M::T> S0,
+__global__ void __launch_bounds__(256) k_step_persistent(const __grid_constant__ Params P, Streams<typename M::T> S0,
                                                          Streams<typename M::T> S1, int steps, GridBarrier* bar,
                                                          unsigned expected, unsigned long long timeout_ns)
 {
@@ -866,7 +866,7 @@ __device__ __forceinline__ void collide_single(const Params& P, const Streams<ty
 
 // Step from PRE: S.src holds the buffer base pointers (direction d at S.src[d]).
 template <class M, int FM, int OUT>
-__global__ void __launch_bounds__(256) k_collide_local(Params P, Streams<typename M::T> S,
+__global__ void __launch_bounds__(256) k_collide_local(const __grid_constant__ Params P, Streams<typename M::T> S,
                                                        Outputs<typename M::C> out)
 {
     if constexpr ((OUT & OUT_SUMS) != 0) reduce_prev(out);
