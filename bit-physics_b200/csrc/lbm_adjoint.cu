@@ -3,6 +3,7 @@
 // no bit-exactness (the forward states it reads are recomputed by the step
 // kernels themselves).
 #include "lbm_adjoint.cuh"
+#include "lbm_compact.cuh"
 #include "lbm_launch.h"
 
 // Threads per block of the per-cell adjoint level kernels.
@@ -24,15 +25,17 @@ __global__ void k_check_unit_interval(const float* __restrict__ a, int n, int* _
     if (i < n && !(a[i] >= 0.0f && a[i] <= 1.0f)) *flag = 1;
 }
 
-__global__ void k_list_special(Params P, int* __restrict__ list, int* __restrict__ count)
-{
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= P.n) return;
-    int x, y, z;
-    decode_xyz(P, idx, x, y, z);
-    const int fl = P.has_flags ? (int)P.flags[idx] : 0;
-    if ((fl & 3) != CELL_SOLID && adj_special(P, idx, x, y, z, fl)) list[atomicAdd(count, 1)] = idx;
-}
+// Kind 0: the special non-solid cells.
+struct SpecialCell {
+    Params P;
+    __device__ int operator()(int idx) const
+    {
+        int x, y, z;
+        decode_xyz(P, idx, x, y, z);
+        const int fl = P.has_flags ? (int)P.flags[idx] : 0;
+        return (fl & 3) != CELL_SOLID && adj_special(P, idx, x, y, z, fl) ? 0 : -1;
+    }
+};
 
 namespace {
 
@@ -91,14 +94,13 @@ cudaError_t launch_adjoint_level(int storage, int force_mode, int level, const A
 
 size_t adjoint_elem_bytes(int storage) { return storage == STORAGE_F64 ? sizeof(double) : sizeof(float); }
 
-cudaError_t launch_list_special(const Params& P, int* list, int* count, cudaStream_t s)
+cudaError_t launch_list_special(const Params& P, int* list, cudaStream_t s)
 {
-    const int block = 256;
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
-    k_list_special<<<grid_for(P.n, block), block, 0, s>>>(P, list, count);
-    return cudaGetLastError();
+    int* count = list + P.n;
+    return compact<1>(SpecialCell{P}, P.n, list, 0, count, count + 1, s);
 }
+
+size_t special_list_ints(int n) { return (size_t)n + 1 + compact_scratch(n, 1); }
 
 cudaError_t launch_widen(const float* in, double* out, size_t count, cudaStream_t s)
 {

@@ -308,10 +308,6 @@ __device__ __forceinline__ bool adj_special(const Params& P, int idx, int x, int
     return (P.flags[idx + (xo - x) * P.nynz] & 3) == CELL_OUTFLOW;
 }
 
-// List of the special non-solid cells (order unspecified; each cell's work
-// is independent of the others').
-__global__ void k_list_special(Params P, int* __restrict__ list, int* __restrict__ count);
-
 // One adjoint level (INIT or STEP) over the plain cells.  S.src: the stored
 // state P_{k-1}.
 template <class M, int FM, int LEVEL>

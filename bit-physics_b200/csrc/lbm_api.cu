@@ -1,6 +1,7 @@
 // lbm_api.cu -- the C ABI of include/lbm_d3q19.h: lattice handles, state
 // transfer, the step loop and the stateless reference functions.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -51,6 +52,16 @@ int cuda_fail(cudaError_t e, const char* what)
         return fail(LBM_ERR_NOMEM, "%s: %s", what, cudaGetErrorString(e));
     }
     return fail(LBM_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+}
+
+cudaError_t device_alloc(void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && drop_arenas(0)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 }  // namespace api
@@ -244,23 +255,11 @@ int refresh_rule_quads(lbm_lattice* h)
 {
     if (h->vec != 4) return LBM_OK;
     const int cap = h->n / 4;
-    int* counts = h->rule_quads + (size_t)QUAD_KINDS * cap;
-    CK(launch_list_rule_quads(h->P, h->rule_quads, cap, counts, h->stream), "rule quad lists");
-    CK(cudaMemcpyAsync(h->rule_counts, counts, sizeof(int) * QUAD_KINDS, cudaMemcpyDeviceToHost, h->stream),
+    CK(launch_list_rule_quads(h->P, h->rule_quads, h->stream), "rule quad lists");
+    CK(cudaMemcpyAsync(h->rule_counts, h->rule_quads + (size_t)QUAD_KINDS * cap, sizeof(int) * QUAD_KINDS,
+                       cudaMemcpyDeviceToHost, h->stream),
        "rule quad counts");
     CK(cudaStreamSynchronize(h->stream), "rule quad sync");
-    // The lists come out in the order of the listing kernel's atomics; in
-    // lattice order, the consecutive tasks of a warp step neighbouring quads,
-    // whose gathers share cache lines.
-    std::vector<int> list;
-    for (int k = 0; k < QUAD_KINDS; ++k) {
-        if (h->rule_counts[k] < 2) continue;
-        int* dev = h->rule_quads + (size_t)k * cap;
-        list.resize(h->rule_counts[k]);
-        CK(cudaMemcpy(list.data(), dev, sizeof(int) * list.size(), cudaMemcpyDeviceToHost), "rule quad list");
-        std::sort(list.begin(), list.end());
-        CK(cudaMemcpy(dev, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice), "rule quad list");
-    }
     // Leading blocks of k_step4: about 0.7 rule tasks per thread for each
     // wave of resident blocks (4 of 128 threads per SM) the plain quads take,
     // so that the rule blocks finish within the plain ones' time.  Sphere
@@ -287,7 +286,7 @@ int check_no_open_step(const lbm_lattice* h)
 int ensure_staging(lbm_lattice* h)
 {
     if (h->staging) return LBM_OK;
-    CK(cudaMalloc((void**)&h->staging, sizeof(double) * Q * (size_t)h->n), "staging allocation");
+    CK(device_alloc((void**)&h->staging, sizeof(double) * Q * (size_t)h->n), "staging allocation");
     return LBM_OK;
 }
 
@@ -440,7 +439,9 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     if (desc->device < 0 || desc->device >= ndev) return fail(LBM_ERR_INVALID, "device %d out of range", desc->device);
     CK(cudaSetDevice(desc->device), "cudaSetDevice");
 
+    static std::atomic<uint64_t> next_id{1};
     lbm_lattice* h = new lbm_lattice();
+    h->id = next_id++;
     h->desc = *desc;
     h->storage = desc->storage;
     h->n = desc->nx * desc->ny * desc->nz;
@@ -469,12 +470,12 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     h->own_stream = true;
     const size_t pop_bytes = h->elem * Q * (size_t)h->n;
     for (int b = 0; b < 2; ++b) {
-        e = cudaMalloc(&h->buf[b], pop_bytes);
+        e = device_alloc((void**)&h->buf[b], pop_bytes);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "population allocation"));
     }
     const size_t cbytes = h->storage == LBM_STORAGE_F64 ? sizeof(double) : sizeof(float);
-    e = cudaMalloc(&h->rho, cbytes * (size_t)h->n);
-    if (e == cudaSuccess) e = cudaMalloc(&h->u, cbytes * 3 * (size_t)h->n);
+    e = device_alloc((void**)&h->rho, cbytes * (size_t)h->n);
+    if (e == cudaSuccess) e = device_alloc((void**)&h->u, cbytes * 3 * (size_t)h->n);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "readback allocation"));
     // TMA-staged step (on request): shared-memory pipeline for f32-arithmetic
     // storages whose rows are multiples of 16 bytes.  Not the default: on the
@@ -516,9 +517,9 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     h->partial_blocks = grid_for(h->n, h->block);
     if (h->partial_blocks < h->tma_grid) h->partial_blocks = h->tma_grid;
     if (h->partial_blocks < h->sums_grid) h->partial_blocks = h->sums_grid;
-    e = cudaMalloc((void**)&h->partials, sizeof(double) * 2 * 5 * (size_t)h->partial_blocks);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->sums, sizeof(double) * 5);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->err, sizeof(int));
+    e = device_alloc((void**)&h->partials, sizeof(double) * 2 * 5 * (size_t)h->partial_blocks);
+    if (e == cudaSuccess) e = device_alloc((void**)&h->sums, sizeof(double) * 5);
+    if (e == cudaSuccess) e = device_alloc((void**)&h->err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "reduction scratch allocation"));
     if (desc->staging == LBM_STAGING_PERSISTENT) {
@@ -527,12 +528,12 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
             cudaGetLastError();
             return cleanup(fail(LBM_ERR_UNSUPPORTED, "persistent staging needs cooperative launch support"));
         }
-        e = cudaMalloc((void**)&h->bar, sizeof(GridBarrier));
+        e = device_alloc((void**)&h->bar, sizeof(GridBarrier));
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "grid barrier allocation"));
         h->persist = true;
     }
     if (h->vec == 4) {
-        e = cudaMalloc((void**)&h->rule_quads, sizeof(int) * ((size_t)QUAD_KINDS * (h->n / 4) + QUAD_KINDS));
+        e = device_alloc((void**)&h->rule_quads, sizeof(int) * rule_quad_ints(h->n / 4));
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "four-cell step set-up"));
         if (cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, desc->device) != cudaSuccess ||
             h->sms < 1)
@@ -544,26 +545,10 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     // walls: the items on the walled faces first, then the interior (fixed
     // by the periodicity, which does not change after creation).
     if (h->vec <= 2 && desc->periodic != 7) {
-        const size_t items = (size_t)h->n / h->vec;
-        e = cudaMalloc((void**)&h->order, sizeof(int) * (items + 1));
-        if (e == cudaSuccess) e = launch_face_order(h->P, h->vec, h->order, h->order + items, h->stream);
-        int faces = -1;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&faces, h->order + items, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        const int items = h->n / h->vec;
+        e = device_alloc((void**)&h->order, sizeof(int) * face_order_ints(items));
+        if (e == cudaSuccess) e = launch_face_order(h->P, h->vec, h->order, h->stream);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "face order"));
-        const long long bx = desc->nx - 2 * (int)h->P.walled[0], by = desc->ny - 2 * (int)h->P.walled[1],
-                        bz = desc->nz / h->vec - 2 * (int)h->P.walled[2];
-        const long long inner = bx > 0 && by > 0 && bz > 0 ? bx * by * bz : 0;
-        if (faces != (long long)items - inner) return cleanup(fail(LBM_ERR_CUDA, "face order incomplete"));
-        if (faces > 1) {  // the face items into lattice order
-            std::vector<int> list(faces);
-            e = cudaMemcpy(list.data(), h->order, sizeof(int) * list.size(), cudaMemcpyDeviceToHost);
-            if (e == cudaSuccess) {
-                std::sort(list.begin(), list.end());
-                e = cudaMemcpy(h->order, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice);
-            }
-            if (e != cudaSuccess) return cleanup(cuda_fail(e, "face order"));
-        }
     }
     // Rest state f = w_i (rho = 1, u = 0).
     e = launch_feq_init(h->storage, h->P, nullptr, nullptr, h->buf[0], h->stream);
@@ -580,6 +565,7 @@ int lbm_destroy(lbm_lattice* h)
     if (!h) return LBM_OK;
     cudaSetDevice(h->desc.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
+    drop_arenas(h->id);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     void* ptrs[] = {h->buf[0], h->buf[1], h->flags, h->bbmask, h->force, h->poro, h->rho,
                     h->u, h->partials, h->sums, h->staging, h->monitor, h->err, h->diag, h->rule_quads, h->bar,
@@ -713,8 +699,8 @@ int lbm_set_flags(lbm_lattice* h, const uint8_t* flags)
         CK(launch(h, KERNEL_OBSERVE, h->buf[h->cur], nullptr, true, h->staging, nullptr, nullptr, nullptr),
            "state rebuild");
     }
-    if (!h->flags) CK(cudaMalloc((void**)&h->flags, n), "flag allocation");
-    if (!h->bbmask) CK(cudaMalloc((void**)&h->bbmask, sizeof(uint32_t) * n), "mask allocation");
+    if (!h->flags) CK(device_alloc((void**)&h->flags, n), "flag allocation");
+    if (!h->bbmask) CK(device_alloc((void**)&h->bbmask, sizeof(uint32_t) * n), "mask allocation");
     CK(cudaMemcpyAsync(h->flags, flags, n, cudaMemcpyHostToDevice, h->stream), "flag upload");
     h->has_flags = true;
     rebuild_params(h);
@@ -737,13 +723,13 @@ int lbm_set_force_field(lbm_lattice* h, const double* force)
         return fail(LBM_ERR_STATE, "lattice was not created with LBM_FORCE_FIELD");
     const size_t cnt = 3 * (size_t)h->n;
     if (h->storage == LBM_STORAGE_F64) {
-        if (!h->force) CK(cudaMalloc(&h->force, sizeof(double) * cnt), "force allocation");
+        if (!h->force) CK(device_alloc((void**)&h->force, sizeof(double) * cnt), "force allocation");
         CK(cudaMemcpyAsync(h->force, force, sizeof(double) * cnt, cudaMemcpyHostToDevice, h->stream), "force upload");
         CK(cudaStreamSynchronize(h->stream), "force sync");
     } else {
         std::vector<float> tmp(cnt);
         for (size_t i = 0; i < cnt; ++i) tmp[i] = (float)force[i];
-        if (!h->force) CK(cudaMalloc(&h->force, sizeof(float) * cnt), "force allocation");
+        if (!h->force) CK(device_alloc((void**)&h->force, sizeof(float) * cnt), "force allocation");
         CK(cudaMemcpyAsync(h->force, tmp.data(), sizeof(float) * cnt, cudaMemcpyHostToDevice, h->stream),
            "force upload");
         CK(cudaStreamSynchronize(h->stream), "force sync");
@@ -764,7 +750,7 @@ int lbm_set_porosity(lbm_lattice* h, const float* alpha)
     for (size_t i = 0; i < n; ++i)
         if (!(alpha[i] >= 0.0f && alpha[i] <= 1.0f))
             return fail(LBM_ERR_INVALID, "porosity at cell %zu is outside [0, 1]", i);
-    if (!h->poro) CK(cudaMalloc((void**)&h->poro, sizeof(float) * n), "porosity allocation");
+    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * n), "porosity allocation");
     CK(cudaMemcpyAsync(h->poro, alpha, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream), "porosity upload");
     CK(cudaStreamSynchronize(h->stream), "porosity sync");
     rebuild_params(h);
@@ -1024,7 +1010,7 @@ int lbm_set_porosity_dev(lbm_lattice* h, const float* alpha)
     CK(cudaMemcpyAsync(&flag, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "flag read");
     CK(cudaStreamSynchronize(h->stream), "porosity check sync");
     if (flag) return fail(LBM_ERR_INVALID, "porosity outside [0, 1] (or NaN)");
-    if (!h->poro) CK(cudaMalloc((void**)&h->poro, sizeof(float) * n), "porosity allocation");
+    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * n), "porosity allocation");
     CK(cudaMemcpyAsync(h->poro, alpha, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream), "porosity copy");
     rebuild_params(h);
     return LBM_OK;
@@ -1070,7 +1056,7 @@ int lbm_step_monitor(lbm_lattice* h, int32_t n_steps, double* sums)
         if (h->monitor) CK(cudaFree(h->monitor), "monitor free");
         h->monitor = nullptr;
         h->monitor_cap = 0;
-        CK(cudaMalloc((void**)&h->monitor, sizeof(double) * 5 * (size_t)n_steps), "monitor allocation");
+        CK(device_alloc((void**)&h->monitor, sizeof(double) * 5 * (size_t)n_steps), "monitor allocation");
         h->monitor_cap = n_steps;
     }
     // Step s writes its per-block partials into one of two buffers; block 0 of
@@ -1181,7 +1167,7 @@ int lbm_diagnostics(lbm_lattice* h, double dx_phys, double* out6)
     if (!out6) return fail(LBM_ERR_INVALID, "null output");
     if (!(dx_phys > 0.0)) return fail(LBM_ERR_INVALID, "dx_phys must be > 0");
     if ((rc = check_force_ready(h))) return rc;
-    if (!h->diag) CK(cudaMalloc((void**)&h->diag, sizeof(double) * (DIAG_SCRATCH + 6)), "diagnostics scratch");
+    if (!h->diag) CK(device_alloc((void**)&h->diag, sizeof(double) * (DIAG_SCRATCH + 6)), "diagnostics scratch");
     if ((rc = observe_rho_u(h, h->rho, h->u))) return rc;
     const double* rho = (const double*)h->rho;
     const double* u = (const double*)h->u;
@@ -1239,7 +1225,7 @@ int workspace(size_t doubles, double** out)
         g_ws.cap = 0;
     }
     if (!g_ws.ptr) {
-        CK(cudaMalloc((void**)&g_ws.ptr, sizeof(double) * doubles), "workspace allocation");
+        CK(device_alloc((void**)&g_ws.ptr, sizeof(double) * doubles), "workspace allocation");
         g_ws.cap = doubles;
         g_ws.device = dev;
     }
@@ -1288,6 +1274,7 @@ extern "C" {
 
 int lbm_release_workspace(void)
 {
+    drop_arenas(0);
     std::lock_guard<std::mutex> lk(g_ws.mu);
     if (g_ws.ptr) cudaFree(g_ws.ptr);
     g_ws.ptr = nullptr;
@@ -1532,7 +1519,7 @@ int batch_build_items(lbm_batch* b)
         if (b->items) CK(cudaFree(b->items), "batch items free");
         b->items = nullptr;
         b->items_cap = 0;
-        CK(cudaMalloc((void**)&b->items, sizeof(BatchItem) * items.size()), "batch items allocation");
+        CK(device_alloc((void**)&b->items, sizeof(BatchItem) * items.size()), "batch items allocation");
         b->items_cap = (int)items.size();
     }
     CK(cudaMemcpy(b->items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice), "items upload");
@@ -1707,7 +1694,7 @@ int lbm_batch_create(const lbm_desc* descs, int32_t count, lbm_batch** out)
     for (lbm_lattice* h : b->lats)
         if ((rc = lbm_set_stream(h, b->stream))) return cleanup(rc);
     b->host_records.resize(count);
-    e = cudaMalloc(&b->records, sizeof(BatchLattice<float>) * count);
+    e = device_alloc((void**)&b->records, sizeof(BatchLattice<float>) * count);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "batch records"));
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
     if (b->sms < 1) b->sms = 1;
@@ -1879,7 +1866,7 @@ int lbm_batch_autotune(lbm_batch* b, int32_t trial_steps, double* best_ms)
         const size_t bytes = h->elem * Q * (size_t)h->n;
         for (int k = 0; k < 2; ++k) {
             void* p = nullptr;
-            cudaError_t e = cudaMalloc(&p, bytes);
+            cudaError_t e = device_alloc((void**)&p, bytes);
             if (e != cudaSuccess) {
                 for (void* q : saved) cudaFree(q);
                 return cuda_fail(e, "autotune snapshot");

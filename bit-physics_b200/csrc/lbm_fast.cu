@@ -1,71 +1,91 @@
 // lbm_fast.cu -- f32-arithmetic step kernels for f32, binary16-shift and
 // bfloat16-shift storage (ModeFast).  Built with multiply-add contraction on.
 #include "lbm_batch.cuh"
+#include "lbm_compact.cuh"
 #include "lbm_kernels.cuh"
 #include "lbm_launch.h"
 
 namespace lbm {
 
-__global__ void k_list_rule_quads(Params P, int* __restrict__ lists, int cap, int* __restrict__ counts)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int idx0 = 4 * q;
-    if (idx0 >= P.n) return;
-    int x, y, z0;
-    decode_xyz(P, idx0, x, y, z0);
-    const uint32_t fl4 = P.has_flags ? *reinterpret_cast<const uint32_t*>(P.flags + idx0) : 0u;
-    const bool face = quad_on_walled_face(P, x, y, z0);
-    if (!face && (fl4 == 0u || fl4 == QUAD_SOLID || fl4 == QUAD_INFLOW)) return;  // k_step4 steps it
-    int kind = QUAD_KIND_OTHER;
-    if (!face) {
+// The list of k_step4's leading blocks that quad q belongs to (QuadKind), or
+// -1 for the quads that the plain path steps.
+struct RuleQuadKind {
+    Params P;
+    __device__ int operator()(int q) const
+    {
+        const int idx0 = 4 * q;
+        int x, y, z0;
+        decode_xyz(P, idx0, x, y, z0);
+        const uint32_t fl4 = P.has_flags ? *reinterpret_cast<const uint32_t*>(P.flags + idx0) : 0u;
+        if (quad_on_walled_face(P, x, y, z0)) return QUAD_KIND_OTHER;
+        if (fl4 == 0u || fl4 == QUAD_SOLID || fl4 == QUAD_INFLOW) return -1;  // k_step4 steps it
         // bytes of four cells, each fluid or solid (near-solid bits allowed)
-        const uint32_t t = fl4 & 0x03030303u;
-        const bool fluid_or_solid = ((t & 0x02020202u) == 0u);
-        if (fluid_or_solid) {
-            kind = QUAD_KIND_NEAR;
-        } else if (fl4 == QUAD_OUTFLOW) {
+        if ((fl4 & 0x02020202u) == 0u) return QUAD_KIND_NEAR;
+        if (fl4 == QUAD_OUTFLOW) {
             const int gx = x == 0 ? P.nx - 1 : x - 1;
             const uint32_t g4 = *reinterpret_cast<const uint32_t*>(P.flags + idx0 + (gx - x) * P.nynz);
-            if (g4 == 0u && !quad_on_walled_face(P, gx, y, z0)) kind = QUAD_KIND_OUTFLOW;
+            if (g4 == 0u && !quad_on_walled_face(P, gx, y, z0)) return QUAD_KIND_OUTFLOW;
         }
+        return QUAD_KIND_OTHER;
     }
-    lists[(size_t)kind * cap + atomicAdd(counts + kind, 1)] = q;
-}
+};
 
-__global__ void k_face_order(Params P, int vec, int* __restrict__ order, int* __restrict__ face_count)
+// Items (of vec cells) on the walled faces are kind 0; the others have their
+// place in the visit order by their rank in the interior box.
+struct FaceItem {
+    Params P;
+    int vec;
+    __host__ __device__ long long inner_items() const
+    {
+        const long long bx = P.nx - 2 * (int)P.walled[0], by = P.ny - 2 * (int)P.walled[1],
+                        bz = P.nz / vec - 2 * (int)P.walled[2];
+        return bx > 0 && by > 0 && bz > 0 ? bx * by * bz : 0;
+    }
+    // rank in the interior box, or -1 for an item on a walled face
+    __device__ int inner_rank(int p) const
+    {
+        const int nzi = P.nz / vec;  // items per row
+        int x, y, z0;
+        decode_xyz(P, p * vec, x, y, z0);
+        const int zi = z0 / vec;
+        const int xo = (int)P.walled[0], yo = (int)P.walled[1], zo = (int)P.walled[2];
+        const int bx = P.nx - 2 * xo, by = P.ny - 2 * yo, bz = nzi - 2 * zo;
+        const bool inner = bx > 0 && by > 0 && bz > 0 && x >= xo && x < P.nx - xo && y >= yo && y < P.ny - yo &&
+                           zi >= zo && zi < nzi - zo;
+        return inner ? ((x - xo) * by + (y - yo)) * bz + (zi - zo) : -1;
+    }
+    __device__ int operator()(int p) const { return inner_rank(p) < 0 ? 0 : -1; }
+};
+
+__global__ void k_inner_order(FaceItem F, int items, int* __restrict__ order)
 {
-    const int nzi = P.nz / vec;  // items per row
-    const int items = P.n / vec;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= items) return;
-    int x, y, z0;
-    decode_xyz(P, p * vec, x, y, z0);
-    const int zi = z0 / vec;
-    const int xo = P.walled[0] ? 1 : 0, yo = P.walled[1] ? 1 : 0, zo = P.walled[2] ? 1 : 0;
-    const int bx = P.nx - 2 * xo, by = P.ny - 2 * yo, bz = nzi - 2 * zo;
-    const bool inner = bx > 0 && by > 0 && bz > 0 && x >= xo && x < P.nx - xo && y >= yo && y < P.ny - yo &&
-                       zi >= zo && zi < nzi - zo;
-    const int n_inner = bx > 0 && by > 0 && bz > 0 ? bx * by * bz : 0;
-    if (inner)
-        order[items - n_inner + ((x - xo) * by + (y - yo)) * bz + (zi - zo)] = p;
-    else
-        order[atomicAdd(face_count, 1)] = p;
+    const int r = F.inner_rank(p);
+    if (r >= 0) order[items - (int)F.inner_items() + r] = p;
 }
 
-cudaError_t launch_face_order(const Params& P, int vec, int* order, int* face_count, cudaStream_t s)
+cudaError_t launch_face_order(const Params& P, int vec, int* order, cudaStream_t s)
 {
-    cudaError_t e = cudaMemsetAsync(face_count, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
-    k_face_order<<<grid_for(P.n / vec, 256), 256, 0, s>>>(P, vec, order, face_count);
-    return cudaGetLastError();
+    const FaceItem F{P, vec};
+    const int items = P.n / vec;
+    int* faces = order + items;
+    k_inner_order<<<grid_for(items, 256), 256, 0, s>>>(F, items, order);
+    return compact<1>(F, items, order, 0, faces, faces + 1, s);
 }
 
-cudaError_t launch_list_rule_quads(const Params& P, int* lists, int cap, int* counts, cudaStream_t s)
+size_t face_order_ints(int items) { return (size_t)items + 1 + compact_scratch(items, 1); }
+
+cudaError_t launch_list_rule_quads(const Params& P, int* lists, cudaStream_t s)
 {
-    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * QUAD_KINDS, s);
-    if (e != cudaSuccess) return e;
-    k_list_rule_quads<<<grid_for(P.n / 4, 256), 256, 0, s>>>(P, lists, cap, counts);
-    return cudaGetLastError();
+    const size_t cap = (size_t)P.n / 4;
+    int* counts = lists + QUAD_KINDS * cap;
+    return compact<QUAD_KINDS>(RuleQuadKind{P}, (int)cap, lists, cap, counts, counts + QUAD_KINDS, s);
+}
+
+size_t rule_quad_ints(int quads)
+{
+    return (size_t)QUAD_KINDS * quads + QUAD_KINDS + compact_scratch(quads, QUAD_KINDS);
 }
 
 // k_step4 over the window's quads, led by the blocks that step the rule quads

@@ -750,16 +750,6 @@ __global__ void __launch_bounds__(128, 4) k_step4(Params P, Streams<typename M::
     }
 }
 
-// The visit order of Params::order for items of `vec` cells (1 or 2): the
-// items on the walled faces first (appended through *face_count), then the
-// others at their rank in the interior box.
-__global__ void k_face_order(Params P, int vec, int* __restrict__ order, int* __restrict__ face_count);
-
-// Lists of the rule quads by kind: quad indices of kind k at lists + k * cap,
-// their number in counts[k] (order unspecified; each quad's work is
-// independent of the others').
-__global__ void k_list_rule_quads(Params P, int* __restrict__ lists, int cap, int* __restrict__ counts);
-
 // ---------------------------------------------------------------------------
 // Many steps in one cooperative launch (lattices that fit in L2)
 // ---------------------------------------------------------------------------

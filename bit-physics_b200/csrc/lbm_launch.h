@@ -65,12 +65,16 @@ cudaError_t launch_feq_init(int storage, const Params& P, const double* rho, con
                             cudaStream_t s);
 cudaError_t launch_mark_near_solid(const Params& P, uint8_t* flags, uint32_t* bbmask, cudaStream_t s);
 // The quads of a lattice (nz a multiple of 4) that k_step4's plain path
-// leaves to its leading blocks, by kind into lists + kind * cap (in no
-// order); their numbers into counts[QUAD_KINDS] (device).
-cudaError_t launch_list_rule_quads(const Params& P, int* lists, int cap, int* counts, cudaStream_t s);
-// Params::order for items of vec (1 or 2) cells; *face_count (device)
-// receives the number of items on the walled faces.
-cudaError_t launch_face_order(const Params& P, int vec, int* order, int* face_count, cudaStream_t s);
+// leaves to its leading blocks, by kind into lists + kind * (n / 4), each in
+// lattice order; behind the lists their numbers (QUAD_KINDS ints) and
+// scratch, rule_quad_ints(n / 4) ints in all.
+cudaError_t launch_list_rule_quads(const Params& P, int* lists, cudaStream_t s);
+size_t rule_quad_ints(int quads);
+// Params::order for items of vec (1 or 2) cells: the items on the walled
+// faces, then the others, each in lattice order; order[items] receives the
+// number of the former, scratch follows (face_order_ints(items) ints in all).
+cudaError_t launch_face_order(const Params& P, int vec, int* order, cudaStream_t s);
+size_t face_order_ints(int items);
 cudaError_t launch_reduce_partials(const double* partials, int nblocks, double* out5, cudaStream_t s);
 // Tier-1 / Tier-2 diagnostics of f64 rho (n) / u (3, n) device arrays into
 // out6 (device): {check_health, rho_min, rho_max, u_max_lat,
@@ -158,8 +162,10 @@ struct AdjointArgs {
 };
 cudaError_t launch_adjoint_level(int storage, int force_mode, int level, const AdjointArgs& a);
 size_t adjoint_elem_bytes(int storage);
-// Compact the special cells of a lattice into list (capacity n), *count on the device.
-cudaError_t launch_list_special(const Params& P, int* list, int* count, cudaStream_t s);
+// The special cells of a lattice in lattice order into list (capacity n),
+// their number at list[n], scratch behind it (special_list_ints(n) ints).
+cudaError_t launch_list_special(const Params& P, int* list, cudaStream_t s);
+size_t special_list_ints(int n);
 cudaError_t launch_widen(const float* in, double* out, size_t count, cudaStream_t s);
 cudaError_t launch_check_unit_interval(const float* a, int n, int* flag, cudaStream_t s);
 

@@ -6,7 +6,8 @@
 // State s_k = the lattice buffer after k steps: s_0 = f_0 (PRE), s_k = P_{k-1}.
 // Memory: ceil(N / K) checkpoints + the final state + K - 1 segment states
 // + two adjoint fields + the special-cell list, all in one device allocation.
-#include <algorithm>
+#include <mutex>
+#include <set>
 #include <vector>
 
 #include "lbm_adjoint.cuh"
@@ -15,13 +16,100 @@
 using namespace lbm;
 using namespace lbm::api;
 
+namespace {
+
+// A destroyed tape leaves its arena with its lattice, and the lattice's next
+// tape takes it when it fits: an optimisation loop runs one tape an iteration
+// on one lattice, and cudaMalloc + cudaFree of the 5 GB of a 128^3 lattice's
+// 100 steps (checkpoints every 25) took 7.2 of the iteration's 30 ms.  At
+// most one arena per lattice and a sixteenth of the GPU's memory in all are
+// kept; destroying the lattice, lbm_release_workspace or any allocation of
+// this library that finds no memory frees them.  No synchronisation is
+// needed: the next tape of the lattice is enqueued on the same stream behind
+// the last use (lbm_set_stream waits for the old stream).
+struct KeptArena {
+    uint64_t owner;
+    int device;
+    void* p;
+    size_t bytes;
+};
+std::mutex g_arena_mu;
+std::vector<KeptArena> g_kept;
+std::set<uint64_t> g_owners;  // lattices that have taped and still exist
+
+size_t kept_limit()
+{
+    static const size_t limit = [] {
+        size_t free_bytes = 0, total = 0;
+        return cudaMemGetInfo(&free_bytes, &total) == cudaSuccess ? total / 16 : (size_t)0;
+    }();
+    return limit;
+}
+
+// The kept arena of the owner when it holds `need` bytes and at most twice
+// that (a smaller or much larger one is freed).
+void* take_arena(uint64_t owner, size_t need, size_t* bytes)
+{
+    std::lock_guard<std::mutex> lk(g_arena_mu);
+    g_owners.insert(owner);
+    for (size_t i = 0; i < g_kept.size(); ++i) {
+        if (g_kept[i].owner != owner) continue;
+        const KeptArena a = g_kept[i];
+        g_kept.erase(g_kept.begin() + i);
+        if (a.bytes >= need && a.bytes <= 2 * need) {
+            *bytes = a.bytes;
+            return a.p;
+        }
+        cudaFree(a.p);
+        break;
+    }
+    return nullptr;
+}
+
+// Keep an arena for its lattice; false: the caller frees it.
+bool keep_arena(const KeptArena& a)
+{
+    std::lock_guard<std::mutex> lk(g_arena_mu);
+    if (!g_owners.count(a.owner)) return false;  // the lattice is gone
+    size_t held = a.bytes;
+    for (const KeptArena& k : g_kept) {
+        if (k.owner == a.owner) return false;
+        held += k.bytes;
+    }
+    if (held > kept_limit()) return false;
+    g_kept.push_back(a);
+    return true;
+}
+
+}  // namespace
+
+bool lbm::api::drop_arenas(uint64_t owner)
+{
+    std::lock_guard<std::mutex> lk(g_arena_mu);
+    int before = 0;
+    bool any = false;
+    if (cudaGetDevice(&before) != cudaSuccess) return false;
+    for (size_t i = g_kept.size(); i-- > 0;) {
+        if (owner && g_kept[i].owner != owner) continue;
+        cudaSetDevice(g_kept[i].device);
+        cudaFree(g_kept[i].p);
+        g_kept.erase(g_kept.begin() + i);
+        any = true;
+    }
+    cudaSetDevice(before);
+    if (owner) g_owners.erase(owner);
+    return any;
+}
+
 struct lbm_tape {
     lbm_lattice* h = nullptr;
+    uint64_t owner = 0;           // the lattice's id
     int device = 0;
     int32_t n_steps = 0;
     int32_t every = 0;
     int params_version = 0;
     void* arena = nullptr;
+    size_t arena_bytes = 0;
     int64_t bytes = 0;
     size_t state_bytes = 0;       // exact size of one state
     std::vector<void*> ck;        // s_0, s_K, s_2K, ...
@@ -44,8 +132,7 @@ void free_tape(lbm_tape* t)
 {
     if (!t) return;
     cudaSetDevice(t->device);
-    if (t->side) cudaStreamSynchronize(t->side);
-    if (t->arena) cudaFree(t->arena);
+    if (t->arena && !keep_arena({t->owner, t->device, t->arena, t->arena_bytes})) cudaFree(t->arena);
     if (t->fork) cudaEventDestroy(t->fork);
     if (t->join) cudaEventDestroy(t->join);
     if (t->side) cudaStreamDestroy(t->side);
@@ -89,6 +176,7 @@ int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, 
     const int nck = (n_steps + every - 1) / every;
     lbm_tape* t = new lbm_tape();
     t->h = h;
+    t->owner = h->id;
     t->device = h->desc.device;
     t->n_steps = n_steps;
     t->every = every;
@@ -103,9 +191,14 @@ int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, 
     const size_t sb = round_up(t->state_bytes, 256);
     const size_t lb = round_up(adjoint_elem_bytes(h->storage) * Q * (size_t)h->n, 256);
     const size_t nstates = (size_t)nck + 1 + (size_t)(every - 1);
-    const size_t listb = round_up(sizeof(int) * ((size_t)h->n + 1), 256);
+    const size_t listb = round_up(sizeof(int) * special_list_ints(h->n), 256);
     const size_t total = nstates * sb + 2 * lb + listb;
-    cudaError_t e = cudaMalloc(&t->arena, total);
+    cudaError_t e = cudaSuccess;
+    t->arena = take_arena(h->id, total, &t->arena_bytes);
+    if (!t->arena) {
+        e = device_alloc(&t->arena, total);
+        t->arena_bytes = total;
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         free_tape(t);
@@ -122,19 +215,10 @@ int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, 
     t->lam[0] = p;
     t->lam[1] = p + lb;
     t->special = (int*)(p + 2 * lb);
-    int* count = t->special + h->n;
-    e = launch_list_special(h->P, t->special, count, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&t->n_special, count, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+    e = launch_list_special(h->P, t->special, h->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&t->n_special, t->special + h->n, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e == cudaSuccess && t->n_special > 1) {
-        // into lattice order: neighbouring cells in a warp's consecutive tasks
-        std::vector<int> cells(t->n_special);
-        e = cudaMemcpy(cells.data(), t->special, sizeof(int) * cells.size(), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) {
-            std::sort(cells.begin(), cells.end());
-            e = cudaMemcpy(t->special, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice);
-        }
-    }
     if (e != cudaSuccess) {
         free_tape(t);
         return cuda_fail(e, "special-cell list");
