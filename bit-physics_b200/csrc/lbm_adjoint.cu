@@ -45,7 +45,7 @@ cudaError_t launch_level_m(int level, const AdjointArgs& a)
     using T = typename M::T;
     using C = typename M::C;
     AdjIO<C> io{(const C*)a.Lin, (C*)a.Lout, a.grad_rho, a.grad_u, a.dalpha, a.grad_f0};
-    const Streams<T> S = make_streams<T>(a.src, nullptr, a.P.n);
+    const Streams<T> S = make_streams<T>(a.src, nullptr, a.P.stride);
     const int block = LBM_ADJ_BLOCK;
     const int grid = grid_for(a.P.n, block);
     const int sb = 128, sg = grid_for(a.n_special, sb);

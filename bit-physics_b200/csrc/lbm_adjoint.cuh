@@ -123,10 +123,10 @@ __device__ __forceinline__ void adj_body_force(const Params& P, int cell, C& Fx,
     } else if constexpr (FM == FORCE_FIELD) {
         if constexpr (std::is_same<C, double>::value) {
             const double* F = (const double*)P.force;
-            Fx = F[cell]; Fy = F[P.n + cell]; Fz = F[2 * P.n + cell];
+            Fx = F[cell]; Fy = F[P.force_stride + cell]; Fz = F[2 * P.force_stride + cell];
         } else {
             const float* F = (const float*)P.force;
-            Fx = F[cell]; Fy = F[P.n + cell]; Fz = F[2 * P.n + cell];
+            Fx = F[cell]; Fy = F[P.force_stride + cell]; Fz = F[2 * P.force_stride + cell];
         }
     } else {
         Fx = Fy = Fz = C(0);

@@ -121,6 +121,7 @@ void init_geometry(Params& P, int nx, int ny, int nz)
     P.n = nx * ny * nz;
     P.cell0 = 0;  // the step kernels' window: every cell
     P.cell_end = P.n;
+    P.stride = P.force_stride = P.n;
     P.nynz = ny * nz;
     P.div_nz.init((uint32_t)nz);
     P.div_ny.init((uint32_t)ny);
@@ -143,12 +144,16 @@ bool dims_ok(long long nx, long long ny, long long nz)
 
 namespace {
 
+int round_up4(int n) { return (n + 3) / 4 * 4; }
+
 void rebuild_params(lbm_lattice* h)
 {
     h->params_version += 1;  // any captured step graph is stale now
     Params& P = h->P;
     const lbm_desc& d = h->desc;
     init_geometry(P, d.nx, d.ny, d.nz);
+    P.stride = h->stride;
+    P.force_stride = h->storage == LBM_STORAGE_F64 ? h->n : round_up4(h->n);
     P.periodic = d.periodic & 7;
     for (int a = 0; a < 3; ++a) P.walled[a] = (P.periodic >> a) & 1 ? 0u : 1u;
     P.has_flags = h->has_flags ? 1 : 0;
@@ -236,6 +241,7 @@ cudaError_t lbm::api::launch(lbm_lattice* h, int kernel, const void* src, void* 
     a.rule_quads = h->rule_quads;
     for (int k = 0; k < QUAD_KINDS; ++k) a.rule_counts[k] = h->rule_counts[k];
     a.rules_grid = h->rules_grid;
+    a.flat = h->flat4 && h->flat_on;
     if (kernel == KERNEL_STEP && !rho && !u && !partials) a.P.order = h->order;
     if (kernel == KERNEL_STEP && h->use_tma) {
         a.tma_grid = h->tma_grid;
@@ -248,11 +254,41 @@ cudaError_t lbm::api::launch(lbm_lattice* h, int kernel, const void* src, void* 
 
 namespace {
 
+// The same for a lattice that may step with k_step4_flat (one list), and
+// whether it does: its bits are those of the one-cell kernel, so this is a
+// question of time alone.  f16, us a step, flat quads against one cell per
+// thread: 256x128x127 periodic 69.7 / 85.3, sphere channel 80.0 / 94.5, six
+// walls 82.8 / 138; 96x96x95 15.5 / 17.5, 17.9 / 18.7, 19.5 / 20.5; 80x80x81
+// 10.8 / 11.3, 12.3 / 13.4, 13.4 / 13.4; 64x64x63 7.2 / 7.2, 8.2 / 8.2, 9.8 /
+// 8.7: a lattice of less than a wave of quads has too few threads to hide its
+// loads, and the more of its quads need a rule the later that turns.  Rows of
+// even length step two cells per thread: there the flat quads were slower
+// (200x128x98 periodic 54.4 / 47.1).
+// Leading blocks: `share` rule cells per thread for each wave of plain blocks:
+// channel 16 (256x128x127: 12 94.0, 24 82.3 us), walls alone 12 (8: 99.8, 16:
+// 88.9).
+int refresh_flat_rules(lbm_lattice* h)
+{
+    const int quads = (h->n + 3) / 4;
+    CK(launch_list_flat_rules(h->P, h->rule_quads, h->stream), "rule quad list");
+    CK(cudaMemcpyAsync(h->rule_counts, h->rule_quads + quads, sizeof(int), cudaMemcpyDeviceToHost, h->stream),
+       "rule quad count");
+    CK(cudaStreamSynchronize(h->stream), "rule quad sync");
+    const long long rules = h->rule_counts[0], plain = quads > rules ? quads - rules : 1;
+    h->flat_on = h->n >= 200000 + 6 * 200000 * rules / quads;
+    const long long share = h->has_flags ? 16 : 12;
+    const long long want = rules * share * h->sms / plain + 1;
+    h->rules_grid = rules > 0 ? (int)(want > 4 * h->sms ? 4 * h->sms : want) : 0;
+    h->params_version += 1;  // a captured step graph holds the old count
+    return LBM_OK;
+}
+
 // The quads k_step4's plain path leaves to its leading blocks, from the
 // current flags and walled faces (four-cell lattices only), and the number
 // of those blocks.
 int refresh_rule_quads(lbm_lattice* h)
 {
+    if (h->flat4) return refresh_flat_rules(h);
     if (h->vec != 4) return LBM_OK;
     const int cap = h->n / 4;
     CK(launch_list_rule_quads(h->P, h->rule_quads, h->stream), "rule quad lists");
@@ -446,6 +482,7 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     h->storage = desc->storage;
     h->n = desc->nx * desc->ny * desc->nz;
     h->elem = storage_bytes(desc->storage);
+    h->stride = storage16 ? round_up4(h->n) : h->n;
     // 128-thread blocks: on the 256x128x128 sphere channel f32 39.5 against
     // 38.9 GLUPS with 256, f16 (pipelined) 59.1 against 58.4 (192: 38.7 /
     // 52.4), f64 17.1 against 16.5.
@@ -461,6 +498,8 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
         h->vec = 4;
     else
         h->vec = desc->storage != LBM_STORAGE_F64 && desc->nz % 2 == 0 ? 2 : 1;
+    h->flat4 = storage16 && desc->cells_per_thread == 0 && desc->nz % 2 != 0 && desc->nz >= FLAT_MIN_NZ &&
+               (desc->staging == LBM_STAGING_AUTO || desc->staging == LBM_STAGING_REGISTERS);
     auto cleanup = [&](int code) {
         lbm_destroy(h);
         return code;
@@ -468,7 +507,9 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "stream creation"));
     h->own_stream = true;
-    const size_t pop_bytes = h->elem * Q * (size_t)h->n;
+    // 64 bytes behind the last direction: k_step4_flat reads aligned groups
+    // that may reach past it (the values are not used)
+    const size_t pop_bytes = h->state_bytes() + 64;
     for (int b = 0; b < 2; ++b) {
         e = device_alloc((void**)&h->buf[b], pop_bytes);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "population allocation"));
@@ -532,8 +573,9 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "grid barrier allocation"));
         h->persist = true;
     }
-    if (h->vec == 4) {
-        e = device_alloc((void**)&h->rule_quads, sizeof(int) * rule_quad_ints(h->n / 4));
+    if (h->vec == 4 || h->flat4) {
+        e = device_alloc((void**)&h->rule_quads,
+                         sizeof(int) * (h->flat4 ? flat_rule_ints((h->n + 3) / 4) : rule_quad_ints(h->n / 4)));
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "four-cell step set-up"));
         if (cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, desc->device) != cudaSuccess ||
             h->sms < 1)
@@ -699,7 +741,11 @@ int lbm_set_flags(lbm_lattice* h, const uint8_t* flags)
         CK(launch(h, KERNEL_OBSERVE, h->buf[h->cur], nullptr, true, h->staging, nullptr, nullptr, nullptr),
            "state rebuild");
     }
-    if (!h->flags) CK(device_alloc((void**)&h->flags, n), "flag allocation");
+    if (!h->flags) {
+        // whole words: the quad kernels read four flags at a time
+        CK(device_alloc((void**)&h->flags, (size_t)round_up4(h->n)), "flag allocation");
+        CK(cudaMemsetAsync(h->flags, 0, (size_t)round_up4(h->n), h->stream), "flag clear");
+    }
     if (!h->bbmask) CK(device_alloc((void**)&h->bbmask, sizeof(uint32_t) * n), "mask allocation");
     CK(cudaMemcpyAsync(h->flags, flags, n, cudaMemcpyHostToDevice, h->stream), "flag upload");
     h->has_flags = true;
@@ -727,10 +773,12 @@ int lbm_set_force_field(lbm_lattice* h, const double* force)
         CK(cudaMemcpyAsync(h->force, force, sizeof(double) * cnt, cudaMemcpyHostToDevice, h->stream), "force upload");
         CK(cudaStreamSynchronize(h->stream), "force sync");
     } else {
-        std::vector<float> tmp(cnt);
-        for (size_t i = 0; i < cnt; ++i) tmp[i] = (float)force[i];
-        if (!h->force) CK(device_alloc((void**)&h->force, sizeof(float) * cnt), "force allocation");
-        CK(cudaMemcpyAsync(h->force, tmp.data(), sizeof(float) * cnt, cudaMemcpyHostToDevice, h->stream),
+        const size_t n = (size_t)h->n, fs = (size_t)h->P.force_stride;
+        std::vector<float> tmp(3 * fs, 0.0f);
+        for (size_t a = 0; a < 3; ++a)
+            for (size_t i = 0; i < n; ++i) tmp[a * fs + i] = (float)force[a * n + i];
+        if (!h->force) CK(device_alloc((void**)&h->force, sizeof(float) * tmp.size()), "force allocation");
+        CK(cudaMemcpyAsync(h->force, tmp.data(), sizeof(float) * tmp.size(), cudaMemcpyHostToDevice, h->stream),
            "force upload");
         CK(cudaStreamSynchronize(h->stream), "force sync");
     }
@@ -750,7 +798,7 @@ int lbm_set_porosity(lbm_lattice* h, const float* alpha)
     for (size_t i = 0; i < n; ++i)
         if (!(alpha[i] >= 0.0f && alpha[i] <= 1.0f))
             return fail(LBM_ERR_INVALID, "porosity at cell %zu is outside [0, 1]", i);
-    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * n), "porosity allocation");
+    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * (size_t)round_up4(h->n)), "porosity allocation");
     CK(cudaMemcpyAsync(h->poro, alpha, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream), "porosity upload");
     CK(cudaStreamSynchronize(h->stream), "porosity sync");
     rebuild_params(h);
@@ -914,6 +962,7 @@ int lbm_step_planes(lbm_lattice* h, int32_t x_begin, int32_t x_end)
     a.rule_quads = h->rule_quads;
     for (int k = 0; k < QUAD_KINDS; ++k) a.rule_counts[k] = h->rule_counts[k];
     a.rules_grid = h->rules_grid;
+    a.flat = h->flat4 && h->flat_on;
     cudaError_t e = h->storage == LBM_STORAGE_F64 ? launch_exact(KERNEL_STEP, h->desc.force_mode, a)
                                                   : launch_fast(h->storage, KERNEL_STEP, h->desc.force_mode, a);
     if (e != cudaSuccess) return cuda_fail(e, "plane-range step launch");
@@ -1010,7 +1059,7 @@ int lbm_set_porosity_dev(lbm_lattice* h, const float* alpha)
     CK(cudaMemcpyAsync(&flag, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "flag read");
     CK(cudaStreamSynchronize(h->stream), "porosity check sync");
     if (flag) return fail(LBM_ERR_INVALID, "porosity outside [0, 1] (or NaN)");
-    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * n), "porosity allocation");
+    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * (size_t)round_up4(h->n)), "porosity allocation");
     CK(cudaMemcpyAsync(h->poro, alpha, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream), "porosity copy");
     rebuild_params(h);
     return LBM_OK;
@@ -1147,7 +1196,7 @@ static int plane_copy(lbm_lattice* h, int32_t x, uint32_t dir_mask, void* dev, b
     if (dir_mask == 0 || dir_mask >= (1u << Q)) return fail(LBM_ERR_INVALID, "direction mask 0x%x invalid", dir_mask);
     if ((rc = check_device_ptr(h, dev, "plane buffer"))) return rc;
     const size_t plane = (size_t)h->desc.ny * h->desc.nz * h->elem;
-    CK(launch_plane_copy(h->buf[h->cur], (size_t)h->n * h->elem, (size_t)x * plane, plane, dir_mask, dev, get,
+    CK(launch_plane_copy(h->buf[h->cur], (size_t)h->stride * h->elem, (size_t)x * plane, plane, dir_mask, dev, get,
                          h->stream),
        "plane copy");
     return LBM_OK;
@@ -1618,11 +1667,11 @@ int batch_upload_records(lbm_batch* b)
         lbm_lattice* h = b->lats[i];
         BatchLattice<float>& r = b->host_records[i];
         r.P = h->P;
-        r.S[0] = make_streams<float>(nullptr, nullptr, h->n);
+        r.S[0] = make_streams<float>(nullptr, nullptr, h->stride);
         // the pointer layout does not depend on T: fill as bytes of the storage
         for (int d = 0; d < Q; ++d) {
-            const char* a = (const char*)h->buf[h->cur] + (size_t)d * h->n * h->elem;
-            const char* c = (const char*)h->buf[h->cur ^ 1] + (size_t)d * h->n * h->elem;
+            const char* a = (const char*)h->buf[h->cur] + (size_t)d * h->stride * h->elem;
+            const char* c = (const char*)h->buf[h->cur ^ 1] + (size_t)d * h->stride * h->elem;
             r.S[0].src[d] = (const float*)a;
             r.S[0].dst[d] = (float*)c;
             r.S[1].src[d] = (const float*)c;
@@ -1687,6 +1736,11 @@ int lbm_batch_create(const lbm_desc* descs, int32_t count, lbm_batch** out)
     for (int i = 0; i < count; ++i) {
         lbm_lattice* h = nullptr;
         if ((rc = lbm_create(&descs[i], &h))) return cleanup(rc);
+        // One cell per thread for odd nz (the same bits): beside other
+        // lattices' kernels the flat quads' rule blocks hold SMs that those
+        // would use.  16 f16 cavities of up to 96^3, 20 steps on 8 branches:
+        // 2.10 ms, with flat quads 2.28.
+        h->flat4 = false;
         b->lats.push_back(h);
     }
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -1863,7 +1917,7 @@ int lbm_batch_autotune(lbm_batch* b, int32_t trial_steps, double* best_ms)
     // Save both buffers and the state flags of every lattice.
     std::vector<void*> saved;
     for (lbm_lattice* h : b->lats) {
-        const size_t bytes = h->elem * Q * (size_t)h->n;
+        const size_t bytes = h->state_bytes();
         for (int k = 0; k < 2; ++k) {
             void* p = nullptr;
             cudaError_t e = device_alloc((void**)&p, bytes);
@@ -1933,7 +1987,7 @@ restore_state:
     cudaStreamSynchronize(b->stream);
     for (int i = 0; i < b->count; ++i) {
         lbm_lattice* h = b->lats[i];
-        const size_t bytes = h->elem * Q * (size_t)h->n;
+        const size_t bytes = h->state_bytes();
         for (int k = 0; k < 2; ++k) {
             cudaMemcpyAsync(h->buf[k], saved[2 * i + k], bytes, cudaMemcpyDeviceToDevice, b->stream);
         }

@@ -83,6 +83,11 @@ struct FastDiv {
 // Everything a step kernel needs to know about one lattice; passed by value.
 struct Params {
     int nx, ny, nz, n, nynz;
+    // Elements from one direction of the population array to the next, and
+    // from one component of the force field to the next: n, rounded up to a
+    // multiple of 4 for the 16-bit storages' populations and the f32 force
+    // fields, so that every direction starts 8-byte aligned.
+    int stride, force_stride;
     FastDiv div_nz, div_ny;
     int periodic;      // bit 0 x, 1 y, 2 z
     unsigned walled[3]; // 1 where the axis is not periodic
@@ -226,6 +231,32 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// The same operations on one cell, never contracted: a lane of a packed
+// expression and its scalar form round alike.
+__device__ __forceinline__ float add2(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub2(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float mul2(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// A constant in every lane of V; a / b per lane; a per-cell input of one
+// cell, or packed of an even cell and the next.
+template <class V>
+__device__ __forceinline__ V lanes(float s)
+{
+    if constexpr (std::is_same<V, float2>::value) return bc2(s);
+    else return s;
+}
+__device__ __forceinline__ float div2(float a, float b) { return __fdividef(a, b); }
+__device__ __forceinline__ float2 div2(float2 a, float2 b)
+{
+    return make_float2(__fdividef(a.x, b.x), __fdividef(a.y, b.y));
+}
+__device__ __forceinline__ float2 rho_safe(float2 r) { return make_float2(rho_safe(r.x), rho_safe(r.y)); }
+template <class V>
+__device__ __forceinline__ V ld_cells(const float* p)
+{
+    return __ldg(reinterpret_cast<const V*>(p));
+}
+
 // Two scalar population values (cells z, z + 1 of one direction, stored at
 // unrelated addresses) as deviations.
 template <bool CG = false, class T>
@@ -268,7 +299,7 @@ __device__ __forceinline__ void force_exact(const Params& P, int cell, double mx
         Fx = P.body_force[0]; Fy = P.body_force[1]; Fz = P.body_force[2];
     } else if (FM == FORCE_FIELD) {
         const double* F = (const double*)P.force;
-        Fx = F[cell]; Fy = F[P.n + cell]; Fz = F[2 * P.n + cell];
+        Fx = F[cell]; Fy = F[P.force_stride + cell]; Fz = F[2 * P.force_stride + cell];
     } else if (FM == FORCE_DRAG) {
         double ka = P.drag_k * (double)P.porosity[cell];
         double beta = ka / (1.0 + 0.5 * ka);
@@ -288,7 +319,7 @@ __device__ __forceinline__ void force_fast(const Params& P, int cell, float mx, 
         Fx = P.body_force_f[0]; Fy = P.body_force_f[1]; Fz = P.body_force_f[2];
     } else if (FM == FORCE_FIELD) {
         const float* F = (const float*)P.force;
-        Fx = __ldg(F + cell); Fy = __ldg(F + P.n + cell); Fz = __ldg(F + 2 * P.n + cell);
+        Fx = __ldg(F + cell); Fy = __ldg(F + P.force_stride + cell); Fz = __ldg(F + 2 * P.force_stride + cell);
     } else if (FM == FORCE_DRAG) {
         float ka = P.drag_kf * __ldg(P.porosity + cell);
         float beta = __fdividef(ka, 1.0f + 0.5f * ka);
@@ -617,53 +648,96 @@ struct ModeFast {
     // BGK + Guo in deviation form, opposite directions paired:
     //   feq_i - w_i = w_i (rho_dev + rho (3 cu + 4.5 cu^2 - 1.5 u^2))
     //   S_i = (1 - omega/2) w_i (3 (c_i - u).F + 9 (c_i.u)(c_i.F))
-    template <int FM>
-    static __device__ __forceinline__ void collide(const Params& P, int cell, C* h)
+    // The collision of the lattices that step one cell per thread, written
+    // with explicit roundings so that one cell (V = float) and two packed
+    // ones (V = float2, cell0 even) give the same bits.  sink(d, value) takes
+    // each direction's post-collision value as soon as it is final.
+    template <int FM, class V, class Sink>
+    static __device__ __forceinline__ void collide1(const Params& P, int cell0, V* h, Sink&& sink)
     {
-        float rd = 0.0f, mx = 0.0f, my = 0.0f, mz = 0.0f;
+        auto bc = [](float v) { return lanes<V>(v); };
+        V rd = h[0], mx = h[1], my = h[3], mz = h[5];
 #pragma unroll
-        for (int d = 0; d < Q; ++d) {
-            rd += h[d];
-            if (cx(d) == 1) mx += h[d]; else if (cx(d) == -1) mx -= h[d];
-            if (cy(d) == 1) my += h[d]; else if (cy(d) == -1) my -= h[d];
-            if (cz(d) == 1) mz += h[d]; else if (cz(d) == -1) mz -= h[d];
+        for (int d = 1; d < Q; ++d) rd = add2(rd, h[d]);
+#pragma unroll
+        for (int d = 2; d < Q; ++d) {
+            if (cx(d)) mx = cx(d) > 0 ? add2(mx, h[d]) : sub2(mx, h[d]);
+            if (cy(d) && d > 3) my = cy(d) > 0 ? add2(my, h[d]) : sub2(my, h[d]);
+            if (cz(d) && d > 5) mz = cz(d) > 0 ? add2(mz, h[d]) : sub2(mz, h[d]);
         }
-        float rho = 1.0f + rd;
-        float inv = __fdividef(1.0f, rho_safe(rho));
-        float Fx, Fy, Fz;
-        force_fast<FM>(P, cell, mx, my, mz, Fx, Fy, Fz);
-        float ux, uy, uz;
-        if (FM == FORCE_NONE) {
-            ux = mx * inv; uy = my * inv; uz = mz * inv;
-        } else {
-            ux = (mx + 0.5f * Fx) * inv; uy = (my + 0.5f * Fy) * inv; uz = (mz + 0.5f * Fz) * inv;
+        const V rho = add2(bc(1.0f), rd);
+        const V inv = div2(bc(1.0f), rho_safe(rho));
+        V F[3] = {bc(0.0f), bc(0.0f), bc(0.0f)};
+        const V m[3] = {mx, my, mz};
+        if constexpr (FM == FORCE_UNIFORM) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) F[a] = bc(P.body_force_f[a]);
+        } else if constexpr (FM == FORCE_FIELD) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) F[a] = ld_cells<V>((const float*)P.force + a * P.force_stride + cell0);
+        } else if constexpr (FM == FORCE_DRAG) {
+            const V ka = mul2(bc(P.drag_kf), ld_cells<V>(P.porosity + cell0));
+            const V nbeta = mul2(bc(-1.0f), div2(ka, fma2(bc(0.5f), ka, bc(1.0f))));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) F[a] = fma2(nbeta, m[a], bc(P.body_force_f[a]));
         }
+        V u[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) u[a] = mul2(FM == FORCE_NONE ? m[a] : fma2(bc(0.5f), F[a], m[a]), inv);
         const float om = P.omega;
-        const float usq15 = 1.5f * (ux * ux + uy * uy + uz * uz);
-        const float base = rd - rho * usq15; // rho_dev + rho(-1.5 u^2)
-        float uF3 = 0.0f, pref = 0.0f;
-        if (FM != FORCE_NONE) { uF3 = 3.0f * (ux * Fx + uy * Fy + uz * Fz); pref = P.pref; }
+        const V usq15 = mul2(bc(1.5f), fma2(u[2], u[2], fma2(u[0], u[0], mul2(u[1], u[1]))));
+        const V base = fma2(mul2(bc(-1.0f), rho), usq15, rd);  // rho_dev + rho(-1.5 u^2)
+        V nuF3 = bc(0.0f);
+        if constexpr (FM != FORCE_NONE)
+            nuF3 = mul2(bc(-3.0f), fma2(u[2], F[2], fma2(u[0], F[0], mul2(u[1], F[1]))));
         // rest direction
-        h[0] += om * (wf(0) * base - h[0]) - (FM != FORCE_NONE ? pref * wf(0) * uF3 : 0.0f);
+        const V rest = fma2(bc(wf(0)), base, mul2(bc(-1.0f), h[0]));
+        if constexpr (FM == FORCE_NONE) h[0] = fma2(bc(om), rest, h[0]);
+        else h[0] = add2(h[0], fma2(bc(om), rest, mul2(bc(P.pref * wf(0)), nuF3)));
+        sink(0, h[0]);
+        const V rho45 = mul2(rho, bc(4.5f));
 #pragma unroll
         for (int d = 1; d < Q; d += 2) {
             const int o = d + 1;
-            const float cu = (float)cx(d) * ux + (float)cy(d) * uy + (float)cz(d) * uz;
             const float w = wf(d);
-            const float sym = w * (base + rho * 4.5f * cu * cu);
-            const float asym = w * rho * 3.0f * cu;
-            float hd = h[d] + om * (sym + asym - h[d]);
-            float ho = h[o] + om * (sym - asym - h[o]);
-            if (FM != FORCE_NONE) {
-                const float cF = (float)cx(d) * Fx + (float)cy(d) * Fy + (float)cz(d) * Fz;
-                const float s_sym = pref * w * (9.0f * cu * cF - uF3);
-                const float s_asym = pref * w * 3.0f * cF;
-                hd += s_sym + s_asym;
-                ho += s_sym - s_asym;
+            const V cu = along(d, u);
+            const V sym = mul2(bc(w), fma2(mul2(rho45, cu), cu, base));
+            const V wr3 = mul2(mul2(bc(w), rho), bc(3.0f));
+            V hd = fma2(bc(om), sub2(fma2(wr3, cu, sym), h[d]), h[d]);
+            V ho = fma2(bc(om), sub2(fma2(mul2(bc(-1.0f), wr3), cu, sym), h[o]), h[o]);
+            if constexpr (FM != FORCE_NONE) {
+                const V cF = along(d, F);
+                const float pw = P.pref * w;
+                const V s_sym = mul2(bc(pw), fma2(mul2(bc(9.0f), cu), cF, nuF3));
+                hd = add2(hd, fma2(bc(pw * 3.0f), cF, s_sym));
+                ho = add2(ho, fma2(bc(-(pw * 3.0f)), cF, s_sym));
             }
             h[d] = hd;
             h[o] = ho;
+            sink(d, hd);
+            sink(o, ho);
         }
+    }
+    // c_d . v of an odd direction (its first component is +1)
+    template <class V>
+    static __device__ __forceinline__ V along(int d, const V* v)
+    {
+        switch (d) {
+        case 1: return v[0];
+        case 3: return v[1];
+        case 5: return v[2];
+        case 7: return add2(v[0], v[1]);
+        case 9: return sub2(v[0], v[1]);
+        case 11: return add2(v[0], v[2]);
+        case 13: return sub2(v[0], v[2]);
+        case 15: return add2(v[1], v[2]);
+        default: return sub2(v[1], v[2]);
+        }
+    }
+    template <int FM>
+    static __device__ __forceinline__ void collide(const Params& P, int cell, C* h)
+    {
+        collide1<FM>(P, cell, h, [](int, float) {});
     }
 
     // The same collision for two cells at once (lanes of float2), in packed
@@ -697,8 +771,8 @@ struct ModeFast {
         } else if constexpr (FM == FORCE_FIELD) {
             const float* F = (const float*)P.force;
             Fx = __ldg(reinterpret_cast<const float2*>(F + cell0));
-            Fy = __ldg(reinterpret_cast<const float2*>(F + P.n + cell0));
-            Fz = __ldg(reinterpret_cast<const float2*>(F + 2 * P.n + cell0));
+            Fy = __ldg(reinterpret_cast<const float2*>(F + P.force_stride + cell0));
+            Fz = __ldg(reinterpret_cast<const float2*>(F + 2 * P.force_stride + cell0));
         } else if constexpr (FM == FORCE_DRAG) {
             const float2 a = __ldg(reinterpret_cast<const float2*>(P.porosity + cell0));
             const float2 ka = mul2(bc2(P.drag_kf), a);
@@ -787,8 +861,8 @@ struct ModeFast {
         } else if constexpr (FM == FORCE_FIELD) {
             const float* F = (const float*)P.force;
             Fx = __ldg(reinterpret_cast<const float2*>(F + cell0));
-            Fy = __ldg(reinterpret_cast<const float2*>(F + P.n + cell0));
-            Fz = __ldg(reinterpret_cast<const float2*>(F + 2 * P.n + cell0));
+            Fy = __ldg(reinterpret_cast<const float2*>(F + P.force_stride + cell0));
+            Fz = __ldg(reinterpret_cast<const float2*>(F + 2 * P.force_stride + cell0));
         } else if constexpr (FM == FORCE_DRAG) {
             const float2 a = __ldg(reinterpret_cast<const float2*>(P.porosity + cell0));
             const float2 ka = mul2(bc2(P.drag_kf), a);

@@ -22,7 +22,7 @@ static void launch_step_out(int kernel, const LaunchArgs& a, int grid)
     using T = typename M::T;
     using C = typename M::C;
     Outputs<C> out{(C*)a.rho, (C*)a.u, a.partials, a.prev_partials, a.prev_count, a.prev_sums};
-    const Streams<T> S = make_streams<T>(a.src, a.dst, a.P.n);
+    const Streams<T> S = make_streams<T>(a.src, a.dst, a.P.stride);
     if (kernel == KERNEL_STEP)
         k_step<M, FM, OUT><<<grid, a.block, 0, a.stream>>>(a.P, S, out);
     else
@@ -39,7 +39,7 @@ static cudaError_t launch_exact_fm(int kernel, const LaunchArgs& a)
         Outputs<double> out{(double*)a.rho, (double*)a.u, a.partials, a.prev_partials, a.prev_count, a.prev_sums,
                           a.first, a.count};
         const int ogrid = a.count < 0 ? grid : grid_for(a.count, a.block);
-        k_observe<M, FM><<<ogrid, a.block, 0, a.stream>>>(a.P, make_streams<double>(a.src, nullptr, a.P.n), a.post,
+        k_observe<M, FM><<<ogrid, a.block, 0, a.stream>>>(a.P, make_streams<double>(a.src, nullptr, a.P.stride), a.post,
                                                           a.f_out, out);
         return cudaGetLastError();
     }
@@ -550,6 +550,7 @@ cudaError_t ref_bgk_step(const Params& P, const double* f, const double* force, 
     if (force) {
         Params Q2 = P;
         Q2.force = force;
+        Q2.force_stride = P.n;
         k_ref_bgk_step<FORCE_FIELD><<<grid_for(P.n, REF_BLOCK), REF_BLOCK, 0, s>>>(Q2, f, fout);
     } else {
         k_ref_bgk_step<FORCE_NONE><<<grid_for(P.n, REF_BLOCK), REF_BLOCK, 0, s>>>(P, f, fout);

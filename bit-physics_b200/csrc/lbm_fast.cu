@@ -88,6 +88,29 @@ size_t rule_quad_ints(int quads)
     return (size_t)QUAD_KINDS * quads + QUAD_KINDS + compact_scratch(quads, QUAD_KINDS);
 }
 
+// Kind 0: the flat quads that k_step4_flat leaves to its leading blocks.
+struct FlatRuleQuad {
+    Params P;
+    __device__ int operator()(int q) const
+    {
+        const int idx0 = 4 * q;
+        int x, y, z0;
+        decode_xyz(P, idx0, x, y, z0);
+        if (flat_quad_split(P, idx0, x, y, z0)) return 0;
+        const uint32_t fl4 = P.has_flags ? *reinterpret_cast<const uint32_t*>(P.flags + idx0) : 0u;
+        return fl4 == 0u || fl4 == QUAD_SOLID || fl4 == QUAD_INFLOW ? -1 : 0;
+    }
+};
+
+cudaError_t launch_list_flat_rules(const Params& P, int* list, cudaStream_t s)
+{
+    const int quads = (P.n + 3) / 4;
+    int* count = list + quads;
+    return compact<1>(FlatRuleQuad{P}, quads, list, 0, count, count + 1, s);
+}
+
+size_t flat_rule_ints(int quads) { return (size_t)quads + 1 + compact_scratch(quads, 1); }
+
 // k_step4 over the window's quads, led by the blocks that step the rule quads
 // (a.rules_grid of them, at most one task per thread).
 template <class M, int FM>
@@ -107,12 +130,30 @@ static cudaError_t launch_step4(const LaunchArgs& a, const Streams<typename M::T
     return cudaGetLastError();
 }
 
+// k_step4_flat over the window's quads, led by the blocks that step the cells
+// of the rule quads (a.rules_grid of them, at most one cell per thread).
+template <class M, int FM>
+static cudaError_t launch_step4_flat(const LaunchArgs& a, const Streams<typename M::T>& S)
+{
+    const int block = a.block < 128 ? a.block : 128;  // the kernel's bound
+    const int first = a.P.cell0 / 4, end = a.P.cell_end < a.P.n ? a.P.cell_end : a.P.n;
+    const int rules = a.rule_counts[0];
+    int rblocks = 0;
+    if (rules > 0) {
+        const int one_each = grid_for(4LL * rules, block);
+        rblocks = a.rules_grid > 0 && a.rules_grid < one_each ? a.rules_grid : one_each;
+    }
+    const int grid = rblocks + grid_for((end + 3) / 4 - first, block);
+    k_step4_flat<M, FM><<<grid, block, 0, a.stream>>>(a.P, S, a.rule_quads, rules, rblocks);
+    return cudaGetLastError();
+}
+
 template <class M, int FM, int OUT>
 static cudaError_t launch_step_out(int kernel, const LaunchArgs& a, int grid)
 {
     using T = typename M::T;
     Outputs<float> out{(float*)a.rho, (float*)a.u, a.partials, a.prev_partials, a.prev_count, a.prev_sums};
-    const Streams<T> S = make_streams<T>(a.src, a.dst, a.P.n);
+    const Streams<T> S = make_streams<T>(a.src, a.dst, a.P.stride);
     if constexpr (sizeof(T) == 2 && OUT == OUT_NONE) {
         if (kernel == KERNEL_STEP && a.vec == 2 && a.pipe_grid > 0) {
             k_step2_pipe<M, FM><<<a.pipe_grid, a.block, 0, a.stream>>>(a.P, S);
@@ -120,6 +161,7 @@ static cudaError_t launch_step_out(int kernel, const LaunchArgs& a, int grid)
             return cudaGetLastError();
         }
         if (kernel == KERNEL_STEP && a.vec == 4) return launch_step4<M, FM>(a, S);
+        if (kernel == KERNEL_STEP && a.flat) return launch_step4_flat<M, FM>(a, S);
     }
     // Steps with readback or sums of a four-cell lattice run the two-cell kernels.
     if constexpr (OUT == OUT_SUMS) {
@@ -154,7 +196,7 @@ static cudaError_t launch_fast_t(int kernel, const LaunchArgs& a)
         Outputs<float> out{(float*)a.rho, (float*)a.u, a.partials, a.prev_partials, a.prev_count, a.prev_sums,
                           a.first, a.count};
         const int ogrid = a.count < 0 ? grid : grid_for(a.count, a.block);
-        k_observe<M, FM><<<ogrid, a.block, 0, a.stream>>>(a.P, make_streams<T>(a.src, nullptr, a.P.n), a.post,
+        k_observe<M, FM><<<ogrid, a.block, 0, a.stream>>>(a.P, make_streams<T>(a.src, nullptr, a.P.stride), a.post,
                                                           a.f_out, out);
         return cudaGetLastError();
     }

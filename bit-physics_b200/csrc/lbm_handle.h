@@ -15,7 +15,9 @@ struct lbm_lattice {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int n = 0;
+    int stride = 0;  // Params::stride
     size_t elem = 0;
+    size_t state_bytes() const { return elem * lbm::Q * (size_t)stride; }  // of a population buffer
     void* buf[2] = {nullptr, nullptr};
     int cur = 0;
     bool pre = true;
@@ -54,6 +56,11 @@ struct lbm_lattice {
     int* rule_quads = nullptr;  // QUAD_KINDS lists of n / 4 entries, then the counts
     int* order = nullptr;       // Params::order of the plain one- / two-cell steps (walled lattices)
     int rule_counts[lbm::QUAD_KINDS] = {0, 0, 0};
+    // k_step4_flat can step the lattice (16-bit storage, odd nz;
+    // rule_quads is then its one list), and does where no outputs are asked
+    // for (refresh_flat_rules).  vec is that of the other steps.
+    bool flat4 = false;
+    bool flat_on = false;
     int rules_grid = 0;
     int rules_grid_set = 0;     // lbm_set_rule_blocks (0: sized from the lists)
     int sms = 148;              // SMs of the lattice's device

@@ -751,6 +751,135 @@ __global__ void __launch_bounds__(128, 4) k_step4(Params P, Streams<typename M::
 }
 
 // ---------------------------------------------------------------------------
+// Four-cell step for 16-bit storage, rows of odd length
+// ---------------------------------------------------------------------------
+
+// Where nz is odd, the quads are four consecutive cells of the
+// flat array (4 q .. 4 q + 3), whatever rows they fall into.  The sources of
+// a direction are then four consecutive elements too, at a distance that only
+// a wrap changes: at a row's end in z two cells need another element (fetched
+// singly and put in its place), and a quad that spans two rows of which one
+// wraps in y is left to the rule blocks, like those on walled faces, those
+// with a rule cell, and the last cells of a lattice of n % 4 != 0 cells.
+// Rows of 5 cells and more: a quad then meets one row end at most.
+constexpr int FLAT_MIN_NZ = 5;
+
+// The quad at cell idx0 = (x, y, z0) cannot be stepped as one piece.
+__device__ __forceinline__ bool flat_quad_split(const Params& P, int idx0, int x, int y, int z0)
+{
+    if (idx0 + 3 >= P.n) return true;
+    if (z0 + 3 < P.nz) return on_walled_face(P, x, y, z0) || on_walled_face(P, x, y, z0 + 3);
+    return y < 1 || y > P.ny - 3 || P.walled[2] || (P.walled[0] && (x == 0 || x == P.nx - 1));
+}
+
+// The fused step of k_step4 over flat quads.  A direction's four sources
+// start at any element of an aligned group of four: one 8-byte and one 4-byte
+// load hold them, and two funnel shifts by the distance to the boundary (the
+// same for a whole warp but where y or x wraps) put them in place.  The
+// leading `rblocks` blocks step the cells of the listed rule quads one by
+// one.  Quads collide as the one-cell kernel does (collide1), bit for bit.
+// Quads that reach out of the window of cells store what lies inside.
+template <class M, int FM>
+__global__ void __launch_bounds__(128, 4)
+    k_step4_flat(const __grid_constant__ Params P, const __grid_constant__ Streams<typename M::T> S,
+                 const int* __restrict__ rules, int n_rules, int rblocks)
+{
+    using T = typename M::T;
+    static_assert(sizeof(T) == 2, "k_step4_flat: 16-bit storage only");
+    const int end = P.cell_end < P.n ? P.cell_end : P.n;
+    if ((int)blockIdx.x < rblocks) {
+        const Outputs<float> none{nullptr, nullptr, nullptr};
+#pragma unroll 1
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 4 * n_rules; k += rblocks * blockDim.x) {
+            const int idx = 4 * __ldg(rules + (k >> 2)) + (k & 3);
+            if (idx >= P.cell0 && idx < end) step_single<M, FM, OUT_NONE>(P, S, none, idx, nullptr);
+        }
+        return;
+    }
+    const int idx0 = (P.cell0 & ~3) + 4 * ((blockIdx.x - rblocks) * blockDim.x + threadIdx.x);
+    if (idx0 >= end) return;
+    int x, y, z0;
+    decode_xyz(P, idx0, x, y, z0);
+    if (flat_quad_split(P, idx0, x, y, z0)) return;  // also keeps every load below within the buffer
+    const Nbr nb0 = make_nbr(P, x, y, z0);
+    // positions in the quad of the row's last cell and of the cell after it
+    // (z = 0, also where the quad starts a row); 4 and more: none
+    const int je = P.nz - 1 - z0;
+    const int jz = z0 == 0 ? 0 : (je < 3 ? je + 1 : 4);
+    uint2 ra[Q];
+    uint32_t rb[Q], edge[Q];
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+        const unsigned short* base = reinterpret_cast<const unsigned short*>(S.src[d]);
+        const int p = nb0.X[1 - cx(d)] + nb0.Y[1 - cy(d)] + z0 - cz(d);
+        const int hi = p & 2;
+        const int a = p & ~3;
+        ra[d] = __ldg(reinterpret_cast<const uint2*>(base + a + 2 * hi));
+        rb[d] = __ldg(reinterpret_cast<const uint32_t*>(base + a + 4 - hi));
+        edge[d] = 0u;
+        if (cz(d) == 1 && jz < 4) edge[d] = __ldg(base + p + jz + P.nz);
+        if (cz(d) == -1 && je < 4) edge[d] = __ldg(base + p + je - P.nz);
+    }
+    const uint32_t fl4 = P.has_flags ? __ldg(reinterpret_cast<const uint32_t*>(P.flags + idx0)) : 0u;
+    if (fl4 != 0u && fl4 != QUAD_SOLID && fl4 != QUAD_INFLOW) return;  // a rule quad: the leading blocks
+    const bool whole = idx0 >= P.cell0 && idx0 + 4 <= end;
+    auto put = [&](int d, uint32_t lo, uint32_t hi) {
+        unsigned short* q = reinterpret_cast<unsigned short*>(S.dst[d]) + idx0;
+        if (whole) {
+            *reinterpret_cast<uint2*>(q) = make_uint2(lo, hi);
+        } else {
+            for (int j = 0; j < 4; ++j)
+                if (idx0 + j >= P.cell0 && idx0 + j < end)
+                    q[j] = (unsigned short)((j < 2 ? lo : hi) >> (16 * (j & 1)));
+        }
+    };
+    if (fl4 == QUAD_SOLID) {  // four solid cells: the rest state
+#pragma unroll
+        for (int d = 0; d < Q; ++d) {
+            const float2 sv = M::shift2(P, d, make_float2(0.0f, 0.0f));
+            const uint32_t w = pack_dev2(sv.x, sv.y, T{});
+            put(d, w, w);
+        }
+        return;
+    }
+    const bool inflow4 = fl4 == QUAD_INFLOW;
+    // byte selections that put an edge value at its position in the quad
+    const uint32_t zl = jz == 0 ? 0x3254u : (jz == 1 ? 0x5410u : 0x3210u);
+    const uint32_t zh = jz == 2 ? 0x3254u : (jz == 3 ? 0x5410u : 0x3210u);
+    const uint32_t el = je == 0 ? 0x3254u : (je == 1 ? 0x5410u : 0x3210u);
+    const uint32_t eh = je == 2 ? 0x3254u : (je == 3 ? 0x5410u : 0x3210u);
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+        const int p = nb0.X[1 - cx(d)] + nb0.Y[1 - cy(d)] + z0 - cz(d);
+        const bool hi = (p & 2) != 0;
+        const uint32_t t0 = hi ? rb[d] : ra[d].x, t1 = hi ? ra[d].x : ra[d].y, t2 = hi ? ra[d].y : rb[d];
+        const unsigned r = 16u * (unsigned)(p & 1);
+        uint32_t lo = __funnelshift_r(t0, t1, r), up = __funnelshift_r(t1, t2, r);
+        if (cz(d) == 1) {
+            lo = __byte_perm(lo, edge[d], zl);
+            up = __byte_perm(up, edge[d], zh);
+        } else if (cz(d) == -1) {
+            lo = __byte_perm(lo, edge[d], el);
+            up = __byte_perm(up, edge[d], eh);
+        }
+        ra[d] = make_uint2(lo, up);
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float2 h[Q];
+#pragma unroll
+        for (int d = 0; d < Q; ++d)
+            h[d] = inflow4 ? bc2(P.inflow_h[d]) : M::unshift2(P, d, word_dev2(half == 0 ? ra[d].x : ra[d].y, T{}));
+        M::template collide1<FM>(P, idx0 + 2 * half, h, [&](int d, float2 v) {
+            const float2 s = M::shift2(P, d, v);
+            const uint32_t w = pack_dev2(s.x, s.y, T{});
+            if (half == 0) rb[d] = w;
+            else put(d, rb[d], w);
+        });
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Many steps in one cooperative launch (lattices that fit in L2)
 // ---------------------------------------------------------------------------
 
@@ -917,7 +1046,7 @@ __global__ void k_store_f64(Params P, const double* __restrict__ f, T* __restric
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)Q * P.n) return;
     const int d = (int)(i / (size_t)P.n);
-    st_f64(dst + i, d, f[i], P);
+    st_f64(dst + (size_t)d * P.stride + (i - (size_t)d * P.n), d, f[i], P);
 }
 
 // storage -> f64 array (PRE state read-out).
@@ -927,7 +1056,7 @@ __global__ void k_load_f64(Params P, const T* __restrict__ src, double* __restri
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)Q * P.n) return;
     const int d = (int)(i / (size_t)P.n);
-    f[i] = ld_f64(src + i, d, P);
+    f[i] = ld_f64(src + (size_t)d * P.stride + (i - (size_t)d * P.n), d, P);
 }
 
 // f = feq(rho, u) with the reference's reciprocal form (equilibrium.py:310-322),
@@ -945,7 +1074,7 @@ __global__ void k_feq_init(Params P, const double* __restrict__ rho, const doubl
     for (int d = 0; d < Q; ++d) {
         double cu = (double)cx(d) * ux + (double)cy(d) * uy + (double)cz(d) * uz;
         double feq = P.w[d] * r * (1.0 + cu * P.inv_cs2 + cu * cu * P.inv_two_cs4 - u_sq * P.inv_two_cs2);
-        st_f64(dst + (size_t)d * P.n + c, d, feq, P);
+        st_f64(dst + (size_t)d * P.stride + c, d, feq, P);
     }
 }
 
@@ -954,14 +1083,15 @@ __global__ void k_feq_init(Params P, const double* __restrict__ rho, const doubl
 // mask != 0.
 __global__ void k_mark_near_solid(Params P, uint8_t* __restrict__ flags, uint32_t* __restrict__ bbmask);
 
-// Per-direction base pointers of a population buffer of n cells.
+// Per-direction base pointers of a population buffer whose directions are
+// `stride` elements apart (Params::stride).
 template <class T>
-inline Streams<T> make_streams(const void* src, void* dst, int n)
+inline Streams<T> make_streams(const void* src, void* dst, int stride)
 {
     Streams<T> S;
     for (int d = 0; d < Q; ++d) {
-        S.src[d] = src ? (const T*)src + (size_t)d * n : nullptr;
-        S.dst[d] = dst ? (T*)dst + (size_t)d * n : nullptr;
+        S.src[d] = src ? (const T*)src + (size_t)d * stride : nullptr;
+        S.dst[d] = dst ? (T*)dst + (size_t)d * stride : nullptr;
     }
     return S;
 }

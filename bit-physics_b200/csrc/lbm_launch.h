@@ -42,6 +42,7 @@ struct LaunchArgs {
     const int* rule_quads = nullptr;  // QUAD_KINDS lists of n / 4 entries
     int rule_counts[QUAD_KINDS] = {0, 0, 0};
     int rules_grid = 0;  // leading blocks (0: one task per thread)
+    bool flat = false;   // steps without outputs run k_step4_flat (rule_quads: its one list)
 };
 
 // Output selection of a step launch (OUT_* bits of lbm_kernels.cuh) from the
@@ -70,6 +71,10 @@ cudaError_t launch_mark_near_solid(const Params& P, uint8_t* flags, uint32_t* bb
 // scratch, rule_quad_ints(n / 4) ints in all.
 cudaError_t launch_list_rule_quads(const Params& P, int* lists, cudaStream_t s);
 size_t rule_quad_ints(int quads);
+// The flat quads that k_step4_flat leaves to its leading blocks, in lattice
+// order; their number at list[ceil(n / 4)], scratch behind it.
+cudaError_t launch_list_flat_rules(const Params& P, int* list, cudaStream_t s);
+size_t flat_rule_ints(int quads);
 // Params::order for items of vec (1 or 2) cells: the items on the walled
 // faces, then the others, each in lattice order; order[items] receives the
 // number of the former, scratch follows (face_order_ints(items) ints in all).
@@ -127,8 +132,8 @@ inline cudaError_t persistent_t(const LaunchArgs& a, int steps, GridBarrier* bar
     const int need = (items + block - 1) / block;
     if (grid > need) grid = need;  // no block without work
     Params P = a.P;
-    Streams<T> S0 = make_streams<T>(a.src, a.dst, a.P.n);
-    Streams<T> S1 = make_streams<T>(a.dst, const_cast<void*>(a.src), a.P.n);
+    Streams<T> S0 = make_streams<T>(a.src, a.dst, a.P.stride);
+    Streams<T> S1 = make_streams<T>(a.dst, const_cast<void*>(a.src), a.P.stride);
     unsigned expected = (unsigned)grid + missing;
     void* args[] = {&P, &S0, &S1, &steps, &bar, &expected, &timeout_ns};
     if ((e = cudaMemsetAsync(bar, 0, sizeof(GridBarrier), a.stream)) != cudaSuccess) return e;

@@ -115,6 +115,7 @@ extern "C" int lbm_conservation_noalloc(const double* f, const uint8_t* flags, i
     P.ny = ny;
     P.nz = nz;
     P.n = (int)n;
+    P.stride = P.n;
     P.cell0 = 0;
     P.cell_end = P.n;
     P.nynz = ny * nz;
@@ -129,7 +130,7 @@ extern "C" int lbm_conservation_noalloc(const double* f, const uint8_t* flags, i
     cudaStream_t s = (cudaStream_t)stream;
     Outputs<double> out{nullptr, nullptr, partials};
     k_observe<ModeExact, FORCE_NONE>
-        <<<grid, NOALLOC_BLOCK, 0, s>>>(P, make_streams<double>(f, nullptr, P.n), false, nullptr, out);
+        <<<grid, NOALLOC_BLOCK, 0, s>>>(P, make_streams<double>(f, nullptr, P.stride), false, nullptr, out);
     if ((e = cudaGetLastError()) != cudaSuccess) return set_error(LBM_ERR_CUDA, cudaGetErrorString(e));
     if ((e = launch_reduce_partials(partials, grid, sums5, s)) != cudaSuccess)
         return set_error(LBM_ERR_CUDA, cudaGetErrorString(e));

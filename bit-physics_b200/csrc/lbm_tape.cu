@@ -180,7 +180,7 @@ int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, 
     t->device = h->desc.device;
     t->n_steps = n_steps;
     t->every = every;
-    t->state_bytes = h->elem * Q * (size_t)h->n;
+    t->state_bytes = h->state_bytes();
     cudaError_t es = cudaStreamCreateWithFlags(&t->side, cudaStreamNonBlocking);
     if (es == cudaSuccess) es = cudaEventCreateWithFlags(&t->fork, cudaEventDisableTiming);
     if (es == cudaSuccess) es = cudaEventCreateWithFlags(&t->join, cudaEventDisableTiming);

@@ -86,7 +86,10 @@ typedef struct lbm_desc {
     int32_t block_size;  /* threads per block for the step kernels; 0 = auto */
     int32_t cells_per_thread; /* step kernel: 1; 2 (f32/f16/bf16 storage,
                                  nz even); 4 (f16/bf16 storage, nz a
-                                 multiple of 4, register staging); 0 = auto */
+                                 multiple of 4, register staging); 0 = auto
+                                 (f16/bf16 lattices of odd nz: four cells of
+                                 the flat array where that is faster, with
+                                 the bits of 1) */
     int32_t staging;     /* step kernel input staging: LBM_STAGING_*         */
     double storage_ref_u[3]; /* f16/bf16 storage: populations are held as the
                                 16-bit deviation from feq(1, storage_ref_u)
