@@ -405,6 +405,15 @@ int lbm::api::check_device_ptr(const lbm_lattice* h, const void* p, const char* 
     return LBM_OK;
 }
 
+int lbm::api::read_rho_u(lbm_lattice* h, double* rho, double* u)
+{
+    if (h->storage == LBM_STORAGE_F64)  // writes both fields: the handle's buffer takes the one not asked for
+        return observe_rho_u(h, rho ? rho : h->rho, u ? u : h->u);
+    CK(launch_read(h->storage, h->desc.force_mode, h->P, h->buf[h->cur], !h->pre, rho, u, h->stream),
+       "readback kernel launch");
+    return LBM_OK;
+}
+
 int lbm::api::observe_rho_u(lbm_lattice* h, void* drho, void* du)
 {
     cudaError_t e = launch(h, KERNEL_OBSERVE, h->buf[h->cur], nullptr, !h->pre, nullptr, drho, du, nullptr);
@@ -1018,6 +1027,15 @@ int lbm_get_rho_u(lbm_lattice* h, double* rho, double* u)
     int rc = check_handle(h);
     if (rc) return rc;
     if ((rc = check_force_ready(h))) return rc;
+    if (h->storage != LBM_STORAGE_F64 && ensure_staging(h) == LBM_OK) {
+        const size_t n = (size_t)h->n;
+        double* du = h->staging + (n + 1) / 2 * 2;  // 16-byte aligned, as the readback's wide stores want it
+        if ((rc = read_rho_u(h, rho ? h->staging : nullptr, u ? du : nullptr))) return rc;
+        if (rho) CK(cudaMemcpyAsync(rho, h->staging, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream), "rho copy");
+        if (u) CK(cudaMemcpyAsync(u, du, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream), "u copy");
+        CK(cudaStreamSynchronize(h->stream), "readback sync");
+        return LBM_OK;
+    }
     if ((rc = observe_rho_u(h, h->rho, h->u))) return rc;
     return readback_to_host(h, h->rho, h->u, rho, u);
 }
@@ -1029,16 +1047,7 @@ int lbm_get_rho_u_dev(lbm_lattice* h, double* rho, double* u)
     if ((rc = check_force_ready(h))) return rc;
     if (!rho && !u) return LBM_OK;
     if ((rc = check_device_ptr(h, rho, "rho")) || (rc = check_device_ptr(h, u, "u"))) return rc;
-    const size_t n = (size_t)h->n;
-    if (h->storage == LBM_STORAGE_F64) {
-        // the readback kernel writes both fields; borrow the handle's buffer
-        // for the one not asked for
-        return observe_rho_u(h, rho ? rho : h->rho, u ? u : h->u);
-    }
-    if ((rc = observe_rho_u(h, h->rho, h->u))) return rc;
-    if (rho) CK(launch_widen((const float*)h->rho, rho, n, h->stream), "rho widen");
-    if (u) CK(launch_widen((const float*)h->u, u, 3 * n, h->stream), "u widen");
-    return LBM_OK;
+    return read_rho_u(h, rho, u);
 }
 
 int lbm_set_porosity_dev(lbm_lattice* h, const float* alpha)
@@ -1217,18 +1226,14 @@ int lbm_diagnostics(lbm_lattice* h, double dx_phys, double* out6)
     if (!(dx_phys > 0.0)) return fail(LBM_ERR_INVALID, "dx_phys must be > 0");
     if ((rc = check_force_ready(h))) return rc;
     if (!h->diag) CK(device_alloc((void**)&h->diag, sizeof(double) * (DIAG_SCRATCH + 6)), "diagnostics scratch");
-    if ((rc = observe_rho_u(h, h->rho, h->u))) return rc;
-    const double* rho = (const double*)h->rho;
-    const double* u = (const double*)h->u;
-    if (h->storage != LBM_STORAGE_F64) {
-        // the f32 readback widened to f64, as lbm_get_rho_u hands it out
+    double* rho = (double*)h->rho;
+    double* u = (double*)h->u;
+    if (h->storage != LBM_STORAGE_F64) {  // f64, as lbm_get_rho_u hands it out
         if ((rc = ensure_staging(h))) return rc;
-        const size_t n = (size_t)h->n;
-        CK(launch_widen((const float*)h->rho, h->staging, n, h->stream), "rho widen");
-        CK(launch_widen((const float*)h->u, h->staging + n, 3 * n, h->stream), "u widen");
         rho = h->staging;
-        u = h->staging + n;
+        u = h->staging + ((size_t)h->n + 1) / 2 * 2;
     }
+    if ((rc = read_rho_u(h, rho, u))) return rc;
     CK(launch_diagnostics(h->P, rho, u, dx_phys, h->diag, h->diag + DIAG_SCRATCH, h->stream), "diagnostics");
     CK(cudaMemcpyAsync(out6, h->diag + DIAG_SCRATCH, sizeof(double) * 6, cudaMemcpyDeviceToHost, h->stream),
        "diagnostics copy");

@@ -379,6 +379,49 @@ cudaError_t launch_persistent(int storage, int force_mode, const LaunchArgs& a, 
     }
 }
 
+template <class T, int FM>
+static cudaError_t read_t(const Params& P, const void* src, bool post, double* rho, double* u, cudaStream_t s)
+{
+    using M = ModeFast<T>;
+    const Streams<T> S = make_streams<T>(src, nullptr, P.stride);
+    const int block = 128;
+    // two doubles at a time where the arrays allow it (n is even for even nz)
+    const bool wide = post && P.nz % 2 == 0 && (uintptr_t)rho % 16 == 0 && (uintptr_t)u % 16 == 0;
+    if constexpr (sizeof(T) == 2) {
+        if (wide && P.nz % 4 == 0) {
+            k_read<M, FM, 4><<<grid_for(P.n / 4, block), block, 0, s>>>(P, S, post, rho, u);
+            return cudaGetLastError();
+        }
+    }
+    if (wide) k_read<M, FM, 2><<<grid_for(P.n / 2, block), block, 0, s>>>(P, S, post, rho, u);
+    else k_read<M, FM, 1><<<grid_for(P.n, block), block, 0, s>>>(P, S, post, rho, u);
+    return cudaGetLastError();
+}
+
+template <class T>
+static cudaError_t read_fm(int force_mode, const Params& P, const void* src, bool post, double* rho, double* u,
+                           cudaStream_t s)
+{
+    switch (force_mode) {
+    case FORCE_NONE: return read_t<T, FORCE_NONE>(P, src, post, rho, u, s);
+    case FORCE_UNIFORM: return read_t<T, FORCE_UNIFORM>(P, src, post, rho, u, s);
+    case FORCE_FIELD: return read_t<T, FORCE_FIELD>(P, src, post, rho, u, s);
+    case FORCE_DRAG: return read_t<T, FORCE_DRAG>(P, src, post, rho, u, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_read(int storage, int force_mode, const Params& P, const void* src, bool post, double* rho,
+                        double* u, cudaStream_t s)
+{
+    switch (storage) {
+    case STORAGE_F32: return read_fm<float>(force_mode, P, src, post, rho, u, s);
+    case STORAGE_F16: return read_fm<__half>(force_mode, P, src, post, rho, u, s);
+    case STORAGE_BF16: return read_fm<__nv_bfloat16>(force_mode, P, src, post, rho, u, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 cudaError_t launch_fast(int storage, int kernel, int force_mode, const LaunchArgs& a)
 {
     switch (storage) {

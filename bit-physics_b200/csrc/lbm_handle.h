@@ -108,7 +108,9 @@ cudaError_t launch(lbm_lattice* h, int kernel, const void* src, void* dst, bool 
 // with partials, earlier partials this step's kernel reduces as well).
 int advance(lbm_lattice* h, void* rho, void* u, double* partials, int* blocks = nullptr,
             const PendingSums* prev = nullptr);
-// Readback of the current state into the handle's rho/u buffers.
+// rho / u of the current state as f64 into device arrays (either may be null).
+int read_rho_u(lbm_lattice* h, double* rho, double* u);
+// The same in the storage's arithmetic (f64 / f32), both fields.
 int observe_rho_u(lbm_lattice* h, void* drho, void* du);
 // LBM_OK when p is NULL or device (or managed) memory of the handle's GPU,
 // LBM_ERR_INVALID naming `what` otherwise (a host pointer would fault a kernel).

@@ -666,6 +666,16 @@ __device__ __forceinline__ void rule_pair(const Params& P, const Streams<typenam
     step_pair<M, FM, OUT_NONE>(P, S, none, idx0, nullptr);
 }
 
+// Direction d's sources of cells z0, z0 + 1 (half 0) or z0 + 2, z0 + 3 of a
+// quad, packed, from the aligned row values at z0 .. z0 + 3 and the one
+// beyond that a z-shifted direction needs.
+__device__ __forceinline__ uint32_t quad_half(int d, int half, uint2 raw, uint32_t edge)
+{
+    if (cz(d) == 0) return half == 0 ? raw.x : raw.y;
+    if (cz(d) == 1) return half == 0 ? (raw.x << 16) | edge : __funnelshift_r(raw.x, raw.y, 16);
+    return half == 0 ? __funnelshift_r(raw.x, raw.y, 16) : __funnelshift_r(raw.y, edge, 16);
+}
+
 // Fused step from POST of the plain quads, four cells per thread, 16-bit
 // storage, nz a multiple of 4: the default step kernel of the 16-bit storages
 // when no readback or sums are asked for.  Every direction is one aligned
@@ -736,10 +746,7 @@ __global__ void __launch_bounds__(128, 4) k_step4(Params P, Streams<typename M::
         float2 h[Q];
 #pragma unroll
         for (int d = 0; d < Q; ++d) {
-            uint32_t w;
-            if (cz(d) == 0) w = half == 0 ? raw[d].x : raw[d].y;
-            else if (cz(d) == 1) w = half == 0 ? (raw[d].x << 16) | edge[d] : __funnelshift_r(raw[d].x, raw[d].y, 16);
-            else w = half == 0 ? __funnelshift_r(raw[d].x, raw[d].y, 16) : __funnelshift_r(raw[d].y, edge[d], 16);
+            const uint32_t w = quad_half(d, half, raw[d], edge[d]);
             h[d] = inflow4 ? make_float2(P.inflow_s[d], P.inflow_s[d]) : word_dev2(w, T{});
         }
         M::template collide2s<FM>(P, idx0 + 2 * half, h, [&](int d, float2 v) {
@@ -1034,6 +1041,131 @@ __global__ void __launch_bounds__(256) k_observe(Params P, Streams<typename M::T
         if (out.partials) emit<M, FM, OUT_SUMS>(P, out, idx, solid, f, cons);
     }
     if (out.partials) block_sum5(cons, out.partials + (size_t)blockIdx.x * 5);
+}
+
+// ---------------------------------------------------------------------------
+// rho / u readback of the f32-arithmetic storages as f64
+// ---------------------------------------------------------------------------
+
+// The fields of N (1 or 2) cells from idx0 on, widened, to f64 arrays rho (n)
+// and u (3, n); either may be null.
+template <int N>
+__device__ __forceinline__ void store_fields(const Params& P, int idx0, const float (&v)[4][N], double* rho, double* u)
+{
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        double* dst = a == 0 ? rho : u;
+        if (!dst) continue;
+        dst += idx0 + (a > 0 ? (size_t)(a - 1) * P.n : 0);
+        if constexpr (N == 1) *dst = (double)v[a][0];
+        else *reinterpret_cast<double2*>(dst) = make_double2((double)v[a][0], (double)v[a][1]);
+    }
+}
+
+template <class M, int FM, class F, int N>
+__device__ __forceinline__ void fields_of(const Params& P, int idx, int j, bool fluid, const F& h, float (&v)[4][N])
+{
+    float f[Q], r = 0.0f, u[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int d = 0; d < Q; ++d) f[d] = h[d];
+    if (fluid) M::template readback<FM>(P, idx + j, f, r, u);
+    v[0][j] = r;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a + 1][j] = u[a];
+}
+
+// The pair idx0, idx0 + 1 of a POST state.
+template <class M, int FM>
+__device__ __forceinline__ void read_pair(const Params& P, const Streams<typename M::T>& S, int idx0, double* rho,
+                                          double* u)
+{
+    int x, y, z0;
+    decode_xyz(P, idx0, x, y, z0);
+    int fl0 = 0, fl1 = 0;
+    if (P.has_flags) {
+        const unsigned short both = __ldg(reinterpret_cast<const unsigned short*>(P.flags + idx0));
+        fl0 = both & 0xff;
+        fl1 = both >> 8;
+    }
+    const Nbr nb0 = make_nbr(P, x, y, z0);
+    const int zp1 = z0 + 2 == P.nz ? 0 : z0 + 2;
+    float2 h[Q];
+    gather_pair<M>(P, S, nb0, z0, zp1, h);
+    bool fluid0 = true, fluid1 = true;
+    const bool face = on_walled_face(P, x, y, z0) || on_walled_face(P, x, y, z0 + 1);
+    if ((fl0 | fl1 | (int)face) != 0)
+        resolve_pair<M, false>(P, S, idx0, x, y, z0, fl0, fl1, face, nb0, zp1, h, fluid0, fluid1);
+    float v[4][2];
+    fields_of<M, FM>(P, idx0, 0, fluid0, Lane<0>{h}, v);
+    fields_of<M, FM>(P, idx0, 1, fluid1, Lane<1>{h}, v);
+    store_fields<2>(P, idx0, v, rho, u);
+}
+
+// The readback of k_observe (the same values) written as f64 at once, VEC
+// cells per thread: 1 (any lattice, and the PRE states), 2 (nz even) or 4
+// (16-bit storage, nz a multiple of 4: the plain quads' sources are one
+// 8-byte load a direction, as in k_step4).  Bound by memory: populations in,
+// 32 bytes a cell out.  Against k_observe (one cell per thread, f32 fields)
+// and two widening passes, bf16 512x256x256 channel: 1281 -> 539 us; f16 /
+// f32 256x128x128: 172 -> 82, 158 -> 95 us.
+template <class M, int FM, int VEC>
+__global__ void __launch_bounds__(128, 4)
+    k_read(const __grid_constant__ Params P, const __grid_constant__ Streams<typename M::T> S, bool post, double* rho,
+           double* u)
+{
+    using T = typename M::T;
+    const int idx0 = VEC * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (idx0 >= P.n) return;
+    if constexpr (VEC == 1) {
+        const int fl = P.has_flags ? (int)P.flags[idx0] : 0;
+        float f[Q], v[4][1];
+        bool fluid;
+        if (post) {
+            int x, y, z;
+            decode_xyz(P, idx0, x, y, z);
+            const Nbr nb = make_nbr(P, x, y, z);
+            gather<M>(P, S, nb, f);
+            fluid = resolve_state<M>(P, S, idx0, x, y, z, fl, nb, f);
+        } else {
+            fluid = (fl & 3) != CELL_SOLID;
+#pragma unroll
+            for (int d = 0; d < Q; ++d) f[d] = M::load(P, S.src[d] + idx0, d);
+        }
+        fields_of<M, FM>(P, idx0, 0, fluid, f, v);
+        store_fields<1>(P, idx0, v, rho, u);
+    } else if constexpr (VEC == 2) {
+        read_pair<M, FM>(P, S, idx0, rho, u);
+    } else {
+        int x, y, z0;
+        decode_xyz(P, idx0, x, y, z0);
+        const uint32_t fl4 = P.has_flags ? __ldg(reinterpret_cast<const uint32_t*>(P.flags + idx0)) : 0u;
+        if (fl4 != 0u || quad_on_walled_face(P, x, y, z0)) {
+#pragma unroll 1
+            for (int j = 0; j < 4; j += 2) read_pair<M, FM>(P, S, idx0 + j, rho, u);
+            return;
+        }
+        const Nbr nb0 = make_nbr(P, x, y, z0);
+        const int zr = z0 + 4 == P.nz ? 0 : z0 + 4;
+        uint2 raw[Q];
+        uint32_t edge[Q];
+#pragma unroll
+        for (int d = 0; d < Q; ++d) {
+            const unsigned short* p =
+                reinterpret_cast<const unsigned short*>(S.src[d]) + nb0.X[1 - cx(d)] + nb0.Y[1 - cy(d)];
+            raw[d] = __ldg(reinterpret_cast<const uint2*>(p + z0));
+            edge[d] = cz(d) == 1 ? (uint32_t)__ldg(p + nb0.Z[0]) : (cz(d) == -1 ? (uint32_t)__ldg(p + zr) : 0u);
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float2 h[Q];
+#pragma unroll
+            for (int d = 0; d < Q; ++d) h[d] = M::unshift2(P, d, word_dev2(quad_half(d, half, raw[d], edge[d]), T{}));
+            float v[4][2];
+            fields_of<M, FM>(P, idx0 + 2 * half, 0, true, Lane<0>{h}, v);
+            fields_of<M, FM>(P, idx0 + 2 * half, 1, true, Lane<1>{h}, v);
+            store_fields<2>(P, idx0 + 2 * half, v, rho, u);
+        }
+    }
 }
 
 // Sum per-block partials in a fixed order (one block).

@@ -54,6 +54,10 @@ inline int grid_for(long long work, int block) { return (int)((work + block - 1)
 // Stateful engine kernels.
 cudaError_t launch_exact(int kernel, int force_mode, const LaunchArgs& a);
 cudaError_t launch_fast(int storage, int kernel, int force_mode, const LaunchArgs& a);
+// rho (n) and u (3, n) of a state of the f32-arithmetic storages as f64;
+// either may be null.
+cudaError_t launch_read(int storage, int force_mode, const Params& P, const void* src, bool post, double* rho,
+                        double* u, cudaStream_t s);
 // Grids of the grid-stride two-cell kernels for this storage / force model /
 // block size on the current device (resident blocks per SM x SMs); 0 where
 // the kernel does not apply.  k_step2_pipe: f16 / bf16; k_step2_sums: f32 /
