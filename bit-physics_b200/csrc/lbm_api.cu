@@ -144,7 +144,41 @@ bool dims_ok(long long nx, long long ny, long long nz)
 
 namespace {
 
+void plain_order(Params& P)
+{
+    P.order = nullptr;
+    P.first.on = 0;
+}
+
 int round_up4(int n) { return (n + 3) / 4 * 4; }
+
+// The visit order of a lattice with walls (one- and two-cell kernels).  Face
+// items apart keep the other warps out of the face path, but an end of a row
+// stepped apart from its row costs whole 32-byte sectors, which memory then
+// moves twice, and the ends of f32 and f64 rows are too many of those.  Six
+// walls, us a step, in rows / all faces first / z faces plane by plane:
+//   within L2   f32 64^3 12.1 / 11.3 / 12.3, 80^3 17.1 / 15.0 / 17.2; f64 64^3
+//               15.4 / 14.2 / 16.4; bf16 90^3 25.0 / 17.4 / 19.1; f16 64x64x66
+//               11.3 / 8.4 / 10.4
+//   beyond      f32 96^3 30.8 / 36.9 / 35.9, 256x128x128 112 / 205 / 145; f64
+//               80^3 30.7 / 36.6 / 35.3, 128^3 103 / 158 / 125; f16 128x128x98
+//               57.8 / 45.1 / 42.0
+// Within L2 that is a list, the faces in lattice order (order); tiny f64
+// lattices, a few blocks in all, are left in their rows (32x16x3 with y walls:
+// 2.4 -> 2.1 us).  Beyond, the order is computed (first): a list's load from
+// memory comes before the gather (y walls, f32 128^3: 54.4 -> 52.2 us).  With
+// walls off the z axis it serves f32 and f64 too, unless rows of odd length
+// shift every warp off its cache lines (f32 128x128x127, y walls: 51.5 / 59.5).
+struct VisitOrder {
+    bool list, computed;
+};
+VisitOrder visit_order(const lbm_lattice* h)
+{
+    if (h->desc.periodic == 7 || h->vec > 2) return {false, false};
+    if (2 * h->state_bytes() <= (size_t)100 << 20) return {!(h->elem == 8 && h->n < 16384), false};
+    const bool pairs16 = h->elem == 2 && h->vec == 2;
+    return {false, pairs16 || ((h->desc.periodic & LBM_PERIODIC_Z) && h->desc.nz % 2 == 0)};
+}
 
 void rebuild_params(lbm_lattice* h)
 {
@@ -156,6 +190,8 @@ void rebuild_params(lbm_lattice* h)
     P.force_stride = h->storage == LBM_STORAGE_F64 ? h->n : round_up4(h->n);
     P.periodic = d.periodic & 7;
     for (int a = 0; a < 3; ++a) P.walled[a] = (P.periodic >> a) & 1 ? 0u : 1u;
+    if (visit_order(h).computed) P.first.init(d.nx, d.ny, d.nz / h->vec, P.walled);
+    P.order = h->order;
     P.has_flags = h->has_flags ? 1 : 0;
     P.flags = h->flags;
     P.bbmask = h->bbmask;
@@ -242,7 +278,7 @@ cudaError_t lbm::api::launch(lbm_lattice* h, int kernel, const void* src, void* 
     for (int k = 0; k < QUAD_KINDS; ++k) a.rule_counts[k] = h->rule_counts[k];
     a.rules_grid = h->rules_grid;
     a.flat = h->flat4 && h->flat_on;
-    if (kernel == KERNEL_STEP && !rho && !u && !partials) a.P.order = h->order;
+    if (kernel != KERNEL_STEP || rho || u || partials) plain_order(a.P);
     if (kernel == KERNEL_STEP && h->use_tma) {
         a.tma_grid = h->tma_grid;
         a.tile = h->tile;
@@ -592,14 +628,11 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     }
     rebuild_params(h);
     if (int rc2 = refresh_rule_quads(h)) return cleanup(rc2);
-    // Visit order of the plain one- and two-cell steps on a lattice with
-    // walls: the items on the walled faces first, then the interior (fixed
-    // by the periodicity, which does not change after creation).
-    if (h->vec <= 2 && desc->periodic != 7) {
-        const int items = h->n / h->vec;
-        e = device_alloc((void**)&h->order, sizeof(int) * face_order_ints(items));
+    if (visit_order(h).list) {  // fixed by the periodicity, which does not change after creation
+        e = device_alloc((void**)&h->order, sizeof(int) * face_order_ints(h->n / h->vec));
         if (e == cudaSuccess) e = launch_face_order(h->P, h->vec, h->order, h->stream);
-        if (e != cudaSuccess) return cleanup(cuda_fail(e, "face order"));
+        if (e != cudaSuccess) return cleanup(cuda_fail(e, "visit order"));
+        h->P.order = h->order;
     }
     // Rest state f = w_i (rho = 1, u = 0).
     e = launch_feq_init(h->storage, h->P, nullptr, nullptr, h->buf[0], h->stream);
@@ -950,6 +983,7 @@ int lbm_step_planes(lbm_lattice* h, int32_t x_begin, int32_t x_end)
     // thread, without outputs, over the window's cells.
     LaunchArgs a;
     a.P = h->P;
+    plain_order(a.P);  // the window's cells in their own order
     a.P.cell0 = x_begin * h->desc.ny * h->desc.nz;
     a.P.cell_end = x_end * h->desc.ny * h->desc.nz;
     a.src = h->buf[h->cur];

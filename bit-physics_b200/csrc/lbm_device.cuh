@@ -80,6 +80,57 @@ struct FastDiv {
     }
 };
 
+// Computed visit order of a lattice with walled faces, for items of one or two
+// cells, so that a warp runs either the face path or the plain one: the items
+// on x faces, then those on y faces (the slower ones start first), then plane
+// by plane its z-face items and its others.  Results do not depend on the
+// order.  When it is used: visit_order (lbm_api.cu).
+struct FaceFirst {
+    int on = 0;               // 0: item t is t
+    int nx, ny, nzi;          // items per axis
+    int xo, yo, zo;           // where the others start (1: after a walled face)
+    int by, bz;               // rows per plane and items per row off the walled faces
+    int xf, yf, zf;           // items on x faces; on y faces off those; on z faces per plane
+    int rows, zper;           // y-face rows per plane; z-face items per row
+    FastDiv div_plane, div_rows, div_bz;
+    __host__ void init(int nx_, int ny_, int nzi_, const unsigned* walled)
+    {
+        nx = nx_; ny = ny_; nzi = nzi_;
+        xo = (int)walled[0]; yo = (int)walled[1]; zo = (int)walled[2];
+        auto inside = [](int n, int o) { return n - 2 * o > 0 ? n - 2 * o : 0; };
+        const int bx = inside(nx, xo);
+        by = inside(ny, yo);
+        bz = inside(nzi, zo);
+        rows = ny - by;
+        zper = nzi - bz;
+        xf = (nx - bx) * ny * nzi;
+        yf = bx * rows * nzi;
+        zf = by * zper;
+        div_plane.init(by > 0 ? by * nzi : 1);
+        div_rows.init(rows > 0 ? rows * nzi : 1);
+        div_bz.init(bz > 0 ? bz : 1);
+        on = 1;
+    }
+    __host__ __device__ __forceinline__ int item(int t) const
+    {
+        const int plane = ny * nzi;
+        if (t < xf) return t < plane ? t : t + (nx - 2) * plane;
+        t -= xf;
+        if (t < yf) {
+            const int x = (int)div_rows.div((uint32_t)t), k = t - x * rows * nzi;
+            return (x + xo) * plane + (k < nzi ? k : k + (ny - 2) * nzi);
+        }
+        t -= yf;
+        const int x = (int)div_plane.div((uint32_t)t);
+        int k = t - x * by * nzi;
+        const int base = (x + xo) * plane + yo * nzi;
+        if (k < zf) return zper == 1 ? base + k * nzi : base + (k >> 1) * nzi + ((k & 1) ? nzi - 1 : 0);
+        k -= zf;
+        const int y = (int)div_bz.div((uint32_t)k);
+        return base + y * nzi + (k - y * bz) + zo;
+    }
+};
+
 // Everything a step kernel needs to know about one lattice; passed by value.
 struct Params {
     int nx, ny, nz, n, nynz;
@@ -132,13 +183,9 @@ struct Params {
     // quads, k_collide_local): they advance the cells [cell0, min(n, cell_end)).
     int cell0 = 0, cell_end = 0x7fffffff;
     // Visit order of the plain steps of k_step (cells) and k_step2 (pairs):
-    // item t is order[t], the items on the walled faces first (the slower
-    // ones start first), then the others, so that a warp runs one of the
-    // two paths (results do not depend on the order).  Null: item t is t.
-    // (The persistent kernel deals items to its blocks statically: there
-    // the face items gathered into a few blocks would set each step's time,
-    // so it keeps them spread.)
+    // item t is order[t], else first.item(t) where first.on, else t.
     const int* order = nullptr;
+    FaceFirst first;
 };
 
 // Number of cells in the step kernels' window.

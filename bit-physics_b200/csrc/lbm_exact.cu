@@ -23,7 +23,9 @@ static void launch_step_out(int kernel, const LaunchArgs& a, int grid)
     using C = typename M::C;
     Outputs<C> out{(C*)a.rho, (C*)a.u, a.partials, a.prev_partials, a.prev_count, a.prev_sums};
     const Streams<T> S = make_streams<T>(a.src, a.dst, a.P.stride);
-    if (kernel == KERNEL_STEP)
+    if (kernel == KERNEL_STEP && OUT == OUT_NONE && a.P.first.on)
+        k_step<M, FM, OUT, OUT == OUT_NONE><<<grid, a.block, 0, a.stream>>>(a.P, S, out);
+    else if (kernel == KERNEL_STEP)
         k_step<M, FM, OUT><<<grid, a.block, 0, a.stream>>>(a.P, S, out);
     else
         k_collide_local<M, FM, OUT><<<grid, a.block, 0, a.stream>>>(a.P, S, out);

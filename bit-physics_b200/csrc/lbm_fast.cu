@@ -175,7 +175,10 @@ static cudaError_t launch_step_out(int kernel, const LaunchArgs& a, int grid)
         // at most the kernel's bound (128 threads for 16-bit storage)
         const int block = a.block < Step2Bounds<T>::threads ? a.block : Step2Bounds<T>::threads;
         const int grid2 = grid_for(window_cells(a.P) / 2, block);
-        k_step2<M, FM, OUT><<<grid2, block, 0, a.stream>>>(a.P, S, out);
+        if (OUT == OUT_NONE && a.P.first.on)
+            k_step2<M, FM, OUT, OUT == OUT_NONE><<<grid2, block, 0, a.stream>>>(a.P, S, out);
+        else
+            k_step2<M, FM, OUT><<<grid2, block, 0, a.stream>>>(a.P, S, out);
         if (a.grid_used) *a.grid_used = grid2;
         return cudaGetLastError();
     }

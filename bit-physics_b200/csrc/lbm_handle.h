@@ -54,7 +54,7 @@ struct lbm_lattice {
     // Four-cell steps (vec == 4): the quads that need a boundary rule, stepped
     // by the leading rules_grid blocks of k_step4.
     int* rule_quads = nullptr;  // QUAD_KINDS lists of n / 4 entries, then the counts
-    int* order = nullptr;       // Params::order of the plain one- / two-cell steps (walled lattices)
+    int* order = nullptr;       // Params::order (visit_order)
     int rule_counts[lbm::QUAD_KINDS] = {0, 0, 0};
     // k_step4_flat can step the lattice (16-bit storage, odd nz;
     // rule_quads is then its one list), and does where no outputs are asked

@@ -180,7 +180,9 @@ __device__ __forceinline__ void step_single(const Params& P, const Streams<typen
 // blocks of 256 per SM the f64 kernel runs in 80 registers (93 unbounded,
 // 2 blocks): 17.1 against 14.5 GLUPS on the 256x128x128 sphere channel with
 // 128-thread blocks; f64 results do not depend on it (no contraction).
-template <class M, int FM, int OUT>
+// FIRST: the visit order is computed (Params::first), in a kernel of its own so
+// that the others do not carry its registers.
+template <class M, int FM, int OUT, bool FIRST = false>
 __global__ void __launch_bounds__(256, 3) k_step(const __grid_constant__ Params P, Streams<typename M::T> S, Outputs<typename M::C> out)
 {
     if constexpr ((OUT & OUT_SUMS) != 0) reduce_prev(out);
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(256, 3) k_step(const __grid_constant__ Params 
     if (t < P.n && t < P.cell_end) {
         int idx = t;
         if constexpr (OUT == OUT_NONE)
-            if (P.order) idx = __ldg(P.order + t);
+            idx = FIRST ? P.first.item(t) : (P.order ? __ldg(P.order + t) : t);
         step_single<M, FM, OUT>(P, S, out, idx, cons);
     }
     if constexpr ((OUT & OUT_SUMS) != 0) block_sum5(cons, out.partials + (size_t)blockIdx.x * 5);
@@ -400,7 +402,7 @@ struct Step2Bounds<__nv_bfloat16> {
     static constexpr int threads = 128, blocks = 4;
 };
 
-template <class M, int FM, int OUT>
+template <class M, int FM, int OUT, bool FIRST = false>
 __global__ void __launch_bounds__(Step2Bounds<typename M::T>::threads, Step2Bounds<typename M::T>::blocks)
     k_step2(Params P, Streams<typename M::T> S,
                                                                     Outputs<typename M::C> out)
@@ -418,7 +420,10 @@ __global__ void __launch_bounds__(Step2Bounds<typename M::T>::threads, Step2Boun
         block_sum5(cons, out.partials + (size_t)blockIdx.x * 5);
     } else {
         if (idx0 < P.n && idx0 < P.cell_end)
-            step_pair<M, FM, OUT>(P, S, out, P.order ? 2 * __ldg(P.order + (idx0 >> 1)) : idx0, cons);
+            step_pair<M, FM, OUT>(P, S, out,
+                                  FIRST ? 2 * P.first.item(idx0 >> 1)
+                                        : (P.order ? 2 * __ldg(P.order + (idx0 >> 1)) : idx0),
+                                  cons);
     }
 }
 
