@@ -135,14 +135,14 @@ __device__ __forceinline__ void adj_body_force(const Params& P, int cell, C& Fx,
 
 // lam: lambda_P in, lambda_f out, through the collision at a cell whose
 // pre-collision state has the moments mo (the transpose needs no more of
-// it).  Returns the cell's dL/dalpha term.
+// it) and drag coefficient beta with derivative dbeta.  Returns the cell's
+// dL/dalpha term.
 template <class M, int FM>
 __device__ __forceinline__ double adj_collide(const Params& P, int cell, const CellMoments<typename M::C>& mo,
-                                              typename M::C* lam)
+                                              typename M::C beta, typename M::C dbeta, typename M::C* lam)
 {
     using C = typename M::C;
-    C beta, dbeta, Fbx, Fby, Fbz;
-    adj_beta<C, FM>(P, cell, beta, dbeta);
+    C Fbx, Fby, Fbz;
     adj_body_force<C, FM>(P, cell, Fbx, Fby, Fbz);
     const C rho = mo.rho;
     const C inv = C(1) / rho;
@@ -251,7 +251,9 @@ __device__ __forceinline__ double cell_lambda(const Params& P, const AdjIO<typen
         const int fl = P.has_flags ? (int)P.flags[c] : 0;
         const uint32_t bb = (fl & FLAG_NEAR_SOLID) ? P.bbmask[c] & CW_MASK_BITS : 0u;
         adj_pull<typename M::C>(P, io.Lin, nb, c, x, y, z, bb, lam);
-        return adj_collide<M, FM>(P, c, mo, lam);
+        typename M::C beta, dbeta;
+        adj_beta<typename M::C, FM>(P, c, beta, dbeta);
+        return adj_collide<M, FM>(P, c, mo, beta, dbeta, lam);
     }
 }
 
@@ -309,7 +311,11 @@ __device__ __forceinline__ bool adj_special(const Params& P, int idx, int x, int
 }
 
 // One adjoint level (INIT or STEP) over the plain cells.  S.src: the stored
-// state P_{k-1}.
+// state P_{k-1}.  Bound by memory (f32 drag: 249 bytes a cell).  All loads -- the
+// state, Lambda, alpha, dL/dalpha, the flags -- are issued before anything is
+// decided or computed: with the flags tested first and dL/dalpha read where it
+// is added to, a warp waited for memory three times instead of once (128^3 f32
+// drag channel: 102 -> 96.8 us a level).
 template <class M, int FM, int LEVEL>
 __global__ void __launch_bounds__(256) k_adjoint_plain(Params P, Streams<typename M::T> S, AdjIO<typename M::C> io)
 {
@@ -318,31 +324,37 @@ __global__ void __launch_bounds__(256) k_adjoint_plain(Params P, Streams<typenam
     if (idx >= P.n) return;
     int x, y, z;
     decode_xyz(P, idx, x, y, z);
+    const Nbr nb = make_nbr(P, x, y, z);
+    C lam[Q];
+    if constexpr (LEVEL != ADJ_INIT) {
+#pragma unroll
+        for (int d = 0; d < Q; ++d) lam[d] = __ldg(io.Lin + (size_t)d * P.n + nb.dst(d));
+    }
+    C f[Q];
+#pragma unroll
+    for (int d = 0; d < Q; ++d) f[d] = M::load(P, S.src[d] + nb.src(d), d);
+    C beta, dbeta;
+    if constexpr (LEVEL != ADJ_INIT) adj_beta<C, FM>(P, idx, beta, dbeta);
+    const bool sum_alpha = FM == FORCE_DRAG && io.dalpha;
+    const double before = sum_alpha ? io.dalpha[idx] : 0.0;
     const int fl = P.has_flags ? (int)P.flags[idx] : 0;
     if ((fl & 3) == CELL_SOLID || adj_special(P, idx, x, y, z, fl)) return;
-    const Nbr nb = make_nbr(P, x, y, z);
     CellMoments<C> mo{C(0), C(0), C(0), C(0)};
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
-        const C v = M::load(P, S.src[d] + nb.src(d), d);
+        const C v = f[d];
         mo.rho += v;
         if (cx(d)) mo.mx += C(cx(d)) * v;
         if (cy(d)) mo.my += C(cy(d)) * v;
         if (cz(d)) mo.mz += C(cz(d)) * v;
     }
     if constexpr (M::mass_is_deviation) mo.rho += C(1);
-    C lam[Q];
     double da;
-    if constexpr (LEVEL == ADJ_INIT) {
-        da = adj_seed<M, FM>(P, idx, mo, io.grad_rho, io.grad_u, lam);
-    } else {
-#pragma unroll
-        for (int d = 0; d < Q; ++d) lam[d] = io.Lin[(size_t)d * P.n + nb.dst(d)];
-        da = adj_collide<M, FM>(P, idx, mo, lam);
-    }
+    if constexpr (LEVEL == ADJ_INIT) da = adj_seed<M, FM>(P, idx, mo, io.grad_rho, io.grad_u, lam);
+    else da = adj_collide<M, FM>(P, idx, mo, beta, dbeta, lam);
 #pragma unroll
     for (int d = 0; d < Q; ++d) io.Lout[(size_t)d * P.n + idx] = lam[d];
-    if (FM == FORCE_DRAG && io.dalpha) io.dalpha[idx] += da;
+    if (sum_alpha) io.dalpha[idx] = before + da;
 }
 
 // One adjoint level (INIT or STEP) over the listed special cells: boundary
