@@ -1038,8 +1038,9 @@ int lbm_set_rule_blocks(lbm_lattice* h, int32_t blocks)
 int lbm_get_rule_blocks(const lbm_lattice* h, int32_t* blocks, int32_t* rule_quads)
 {
     if (!h) return fail(LBM_ERR_INVALID, "null lattice handle");
-    if (blocks) *blocks = h->rules_grid;
-    if (rule_quads) *rule_quads = h->rule_counts[0] + h->rule_counts[1] + h->rule_counts[2];
+    const bool four = h->vec == 4;  // flat quads' lists are not reported
+    if (blocks) *blocks = four ? h->rules_grid : 0;
+    if (rule_quads) *rule_quads = four ? h->rule_counts[0] + h->rule_counts[1] + h->rule_counts[2] : 0;
     return LBM_OK;
 }
 

@@ -32,7 +32,7 @@ enum BatchSched : int {
     SCHED_PAIR_SCALAR = 1, // two cells per thread, scalar memory access, f32x2 collision
     SCHED_PAIR_MIXED = 2,  // as 1, but vector access for lattices with an even nz
     SCHED_BRANCHES = 3,    // no batched kernel: each lattice's own step kernels on
-                           // parallel streams, captured into one graph per two steps
+                           // parallel streams, captured into graphs of eight (or two) steps
 };
 
 // First step after a state upload: collide in place, one cell per thread.
