@@ -1729,13 +1729,24 @@ int batch_build_branches(lbm_batch* b, int nb)
 // branches meet at a graph's end only.  A branch of a graph takes its lattices
 // one after the other, each through all the graph's steps, while it sits in
 // L2.  Eight steps against two with a join after each: 16 cavities of up to
-// 96^3 (f16), 20 steps and readbacks, 2.10 -> 1.95 ms.
+// 96^3 (f16), 20 steps and readbacks, 2.10 -> 1.95 ms.  A batch of many times
+// L2 keeps graphs of two steps with a join after each: 64 cavities, 2.5 GB, on 8
+// branches 38.2 GLUPS so and 36.7 in eights.
 constexpr int BRANCH_GRAPH_STEPS[2] = {2, 8};
 constexpr int BRANCH_GRAPH_NODES = 4096;  // more launches than this are not put into one graph
+constexpr size_t BRANCH_GRAPH_BYTES = (size_t)512 << 20;  // nor eight steps of more population bytes
 
-// `steps` steps of every lattice with its own kernels on its branch, forked
-// from and joined into the batch stream.
-cudaError_t batch_branch_steps(lbm_batch* b, int steps, bool by_lattice)
+size_t batch_bytes(const lbm_batch* b)
+{
+    size_t bytes = 0;
+    for (const lbm_lattice* h : b->lats) bytes += 2 * h->state_bytes();
+    return bytes;
+}
+
+// `steps` steps of every lattice, the first of them step `first` from the
+// current buffers, with its own kernels on its branch, forked from and joined
+// into the batch stream.
+cudaError_t batch_branch_steps(lbm_batch* b, int first, int steps, bool by_lattice)
 {
     cudaError_t e;
     if ((e = cudaEventRecord(b->root, b->stream)) != cudaSuccess) return e;
@@ -1744,7 +1755,7 @@ cudaError_t batch_branch_steps(lbm_batch* b, int steps, bool by_lattice)
         if ((e = cudaStreamWaitEvent(b->branches[k], b->root, 0)) != cudaSuccess) return e;
     auto step = [&](int i, int s) {
         lbm_lattice* h = b->lats[i];
-        const int c = h->cur ^ (s & 1);
+        const int c = h->cur ^ ((first + s) & 1);
         cudaStream_t own = h->stream;
         h->stream = b->branches[b->branch_of[i]];
         const cudaError_t r = launch(h, KERNEL_STEP, h->buf[c], h->buf[c ^ 1], false, nullptr, nullptr, nullptr, nullptr);
@@ -1790,7 +1801,13 @@ int capture_branch_graph(lbm_batch* b, int which)
     g.exec = nullptr;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "graph capture begin");
-    const cudaError_t e0 = batch_branch_steps(b, BRANCH_GRAPH_STEPS[which], true);
+    cudaError_t e0;
+    if (which == 0 && batch_bytes(b) > BRANCH_GRAPH_BYTES) {
+        e0 = batch_branch_steps(b, 0, 1, false);
+        if (e0 == cudaSuccess) e0 = batch_branch_steps(b, 1, 1, false);
+    } else {
+        e0 = batch_branch_steps(b, 0, BRANCH_GRAPH_STEPS[which], true);
+    }
     const cudaError_t e1 = cudaStreamEndCapture(b->stream, &graph);
     if (e0 != cudaSuccess || e1 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
@@ -1995,15 +2012,16 @@ int lbm_batch_step(lbm_batch* b, int32_t n_steps)
     const int rest = n_steps - done;
     if (rest <= 0) return LBM_OK;
     if (b->sched == SCHED_BRANCHES) {
-        // Whole graphs of eight steps, the rest launched (a call of fewer steps:
-        // whole graphs of two).
-        const int which = rest >= BRANCH_GRAPH_STEPS[1] && b->count * BRANCH_GRAPH_STEPS[1] <= BRANCH_GRAPH_NODES;
+        // Whole graphs of eight steps, the rest launched (a call of fewer steps, a
+        // large batch: whole graphs of two).
+        const int which = rest >= BRANCH_GRAPH_STEPS[1] && b->count * BRANCH_GRAPH_STEPS[1] <= BRANCH_GRAPH_NODES &&
+                          batch_bytes(b) <= BRANCH_GRAPH_BYTES;
         const int per = BRANCH_GRAPH_STEPS[which];
         if (rest >= per && !branch_graph_current(b, b->branch_graph[which]) && (rc = capture_branch_graph(b, which)))
             return rc;
         for (int k = 0; k + per <= rest; k += per)
             CK(cudaGraphLaunch(b->branch_graph[which].exec, b->stream), "branch graph launch");
-        if (rest % per) CK(batch_branch_steps(b, rest % per, false), "branch step launch");
+        if (rest % per) CK(batch_branch_steps(b, 0, rest % per, false), "branch step launch");
         batch_advance_bookkeeping(b, rest);
         return LBM_OK;
     }
