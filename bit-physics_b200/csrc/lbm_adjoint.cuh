@@ -310,12 +310,21 @@ __device__ __forceinline__ bool adj_special(const Params& P, int idx, int x, int
     return (P.flags[idx + (xo - x) * P.nynz] & 3) == CELL_OUTFLOW;
 }
 
+// Whether k_adjoint_plain issues its loads before the flags are tested.  With
+// drag, the flags tested first and dL/dalpha read where it is added to made a
+// warp wait for memory three times instead of once.  Loads that do not wait for
+// the flags take 80 registers instead of 64, though, which the other force
+// models only earn back in f64 and in f32 without a force field.  us a level
+// and replayed step of a 128^3 channel, before / loads first / flags first: f32
+// drag 171 / 166 / -, none 157 / 155 / 157, field 166 / 183 / 164; f16 none 131
+// / 135 / 128, uniform 130 / 139 / 133, field 143 / 157 / 144.
+template <class M, int FM>
+constexpr bool adj_loads_first = FM == FORCE_DRAG || std::is_same<typename M::T, double>::value ||
+                                 (std::is_same<typename M::T, float>::value && FM != FORCE_FIELD);
+
 // One adjoint level (INIT or STEP) over the plain cells.  S.src: the stored
-// state P_{k-1}.  Bound by memory (f32 drag: 249 bytes a cell).  All loads -- the
-// state, Lambda, alpha, dL/dalpha, the flags -- are issued before anything is
-// decided or computed: with the flags tested first and dL/dalpha read where it
-// is added to, a warp waited for memory three times instead of once (128^3 f32
-// drag channel: 102 -> 96.8 us a level).
+// state P_{k-1}.  Bound by memory (f32 drag: 249 bytes a cell; 96.8 us a level
+// at 128^3).
 template <class M, int FM, int LEVEL>
 __global__ void __launch_bounds__(256) k_adjoint_plain(Params P, Streams<typename M::T> S, AdjIO<typename M::C> io)
 {
@@ -324,37 +333,58 @@ __global__ void __launch_bounds__(256) k_adjoint_plain(Params P, Streams<typenam
     if (idx >= P.n) return;
     int x, y, z;
     decode_xyz(P, idx, x, y, z);
-    const Nbr nb = make_nbr(P, x, y, z);
-    C lam[Q];
-    if constexpr (LEVEL != ADJ_INIT) {
-#pragma unroll
-        for (int d = 0; d < Q; ++d) lam[d] = __ldg(io.Lin + (size_t)d * P.n + nb.dst(d));
-    }
-    C f[Q];
-#pragma unroll
-    for (int d = 0; d < Q; ++d) f[d] = M::load(P, S.src[d] + nb.src(d), d);
-    C beta, dbeta;
-    if constexpr (LEVEL != ADJ_INIT) adj_beta<C, FM>(P, idx, beta, dbeta);
-    const bool sum_alpha = FM == FORCE_DRAG && io.dalpha;
-    const double before = sum_alpha ? io.dalpha[idx] : 0.0;
-    const int fl = P.has_flags ? (int)P.flags[idx] : 0;
-    if ((fl & 3) == CELL_SOLID || adj_special(P, idx, x, y, z, fl)) return;
     CellMoments<C> mo{C(0), C(0), C(0), C(0)};
-#pragma unroll
-    for (int d = 0; d < Q; ++d) {
-        const C v = f[d];
+    auto add_moments = [&](int d, C v) {
         mo.rho += v;
         if (cx(d)) mo.mx += C(cx(d)) * v;
         if (cy(d)) mo.my += C(cy(d)) * v;
         if (cz(d)) mo.mz += C(cz(d)) * v;
+    };
+    C lam[Q], beta, dbeta;
+    if constexpr (adj_loads_first<M, FM>) {
+        const Nbr nb = make_nbr(P, x, y, z);
+        if constexpr (LEVEL != ADJ_INIT) {
+#pragma unroll
+            for (int d = 0; d < Q; ++d) lam[d] = __ldg(io.Lin + (size_t)d * P.n + nb.dst(d));
+        }
+        C f[Q];
+#pragma unroll
+        for (int d = 0; d < Q; ++d) f[d] = M::load(P, S.src[d] + nb.src(d), d);
+        if constexpr (LEVEL != ADJ_INIT) adj_beta<C, FM>(P, idx, beta, dbeta);
+        const bool sum_alpha = FM == FORCE_DRAG && io.dalpha;
+        const double before = sum_alpha ? io.dalpha[idx] : 0.0;
+        const int fl = P.has_flags ? (int)P.flags[idx] : 0;
+        if ((fl & 3) == CELL_SOLID || adj_special(P, idx, x, y, z, fl)) return;
+#pragma unroll
+        for (int d = 0; d < Q; ++d) add_moments(d, f[d]);
+        if constexpr (M::mass_is_deviation) mo.rho += C(1);
+        double da;
+        if constexpr (LEVEL == ADJ_INIT) da = adj_seed<M, FM>(P, idx, mo, io.grad_rho, io.grad_u, lam);
+        else da = adj_collide<M, FM>(P, idx, mo, beta, dbeta, lam);
+        if (sum_alpha) io.dalpha[idx] = before + da;
+    } else {
+        const int fl = P.has_flags ? (int)P.flags[idx] : 0;
+        if ((fl & 3) == CELL_SOLID || adj_special(P, idx, x, y, z, fl)) return;
+        const Nbr nb = make_nbr(P, x, y, z);
+        if constexpr (LEVEL != ADJ_INIT) {
+#pragma unroll
+            for (int d = 0; d < Q; ++d) lam[d] = __ldg(io.Lin + (size_t)d * P.n + nb.dst(d));
+        }
+        C f[Q];
+#pragma unroll
+        for (int d = 0; d < Q; ++d) f[d] = M::load(P, S.src[d] + nb.src(d), d);
+#pragma unroll
+        for (int d = 0; d < Q; ++d) add_moments(d, f[d]);
+        if constexpr (M::mass_is_deviation) mo.rho += C(1);
+        if constexpr (LEVEL == ADJ_INIT) {
+            adj_seed<M, FM>(P, idx, mo, io.grad_rho, io.grad_u, lam);
+        } else {
+            adj_beta<C, FM>(P, idx, beta, dbeta);
+            adj_collide<M, FM>(P, idx, mo, beta, dbeta, lam);
+        }
     }
-    if constexpr (M::mass_is_deviation) mo.rho += C(1);
-    double da;
-    if constexpr (LEVEL == ADJ_INIT) da = adj_seed<M, FM>(P, idx, mo, io.grad_rho, io.grad_u, lam);
-    else da = adj_collide<M, FM>(P, idx, mo, beta, dbeta, lam);
 #pragma unroll
     for (int d = 0; d < Q; ++d) io.Lout[(size_t)d * P.n + idx] = lam[d];
-    if (sum_alpha) io.dalpha[idx] = before + da;
 }
 
 // One adjoint level (INIT or STEP) over the listed special cells: boundary
