@@ -290,16 +290,36 @@ cudaError_t lbm::api::launch(lbm_lattice* h, int kernel, const void* src, void* 
 
 namespace {
 
-// The same for a lattice that may step with k_step4_flat (one list), and
-// whether it does: its bits are those of the one-cell kernel, so this is a
-// question of time alone.  f16, us a step, flat quads against one cell per
-// thread: 256x128x127 periodic 69.7 / 85.3, sphere channel 80.0 / 94.5, six
-// walls 82.8 / 138; 96x96x95 15.5 / 17.5, 17.9 / 18.7, 19.5 / 20.5; 80x80x81
-// 10.8 / 11.3, 12.3 / 13.4, 13.4 / 13.4; 64x64x63 7.2 / 7.2, 8.2 / 8.2, 9.8 /
-// 8.7: a lattice of less than a wave of quads has too few threads to hide its
-// loads, and the more of its quads need a rule the later that turns.  Rows of
-// even length step two cells per thread: there the flat quads were slower
-// (200x128x98 periodic 54.4 / 47.1).
+// Cells from which on a lattice steps with k_step4_flat: its bits are those of
+// the one-cell kernel, so this is a question of time alone.  r: the share of
+// quads that need a rule.  A lattice of less than a wave of quads has too few
+// threads to hide its loads, and the cells of rule quads cost more than one by
+// one in their own kernel: on walled faces (moving-wall products on a chain of
+// loads) a lot, off them (flags alone) little.  Flat quads against one cell per
+// thread, time ratio by cells, f16 without force:
+//   periodic, r < 0.01       0.25 M 1.00, 0.35 M 1.00-1.12, 0.5 M 1.00-1.08, 1 M
+//                            1.06-1.17, 2 M 1.20, 4 M 1.24 (drag 1.44)
+//   spheres, r 0.02-0.07     0.15 M 0.97-1.09, 0.25 M 1.02-1.19, 0.5 M 1.08-1.18,
+//                            1 M 1.10-1.17, 4 M 1.14-1.22
+//   y walls, r 0.01-0.02     0.25 M 1.01-1.13, 0.5 M 1.05-1.13, 1 M 1.17, 4 M 1.41
+//            r 0.03 / 0.05   0.25 M 1.02, 0.36 M 1.00 / 0.35 M 0.94, 0.5 M 1.00
+//            r 0.13          0.25 M 0.89, 0.5 M 0.93, 0.7 M 1.00, 1 M 1.09, 2 M 1.18
+//   six walls, r 0.10        0.7 M 1.06 (0.09: 1 M 1.17)
+//            r 0.15-0.17     0.25 M 0.89, 0.5 M 0.88-1.04, 0.7 M 0.93-1.05, 1 M
+//                            1.05-1.14, 2 M 1.17-1.31
+//            r 0.22          0.7 M 0.95, 1 M 1.00, 2 M 1.21
+//            r 0.56 (nz 9)   1 M 0.78, 2 M 0.98, 4 M 1.03
+// bf16 and the force models lie within a few per cent of these.  Rows of even
+// length step two cells per thread: there the flat quads were slower
+// (200x128x98 periodic 54.4 / 47.1 us).
+double flat_min_cells(const lbm_lattice* h, double r)
+{
+    if (h->desc.periodic != 7) return 230000.0 + 5.2e6 * (r > 0.025 ? r - 0.025 : 0.0);
+    return h->has_flags ? 200000.0 + 1.2e6 * r : 300000.0;
+}
+
+// The same as below for a lattice that may step with k_step4_flat (one list),
+// and whether it does.
 // Leading blocks: `share` rule cells per thread for each wave of plain blocks:
 // channel 16 (256x128x127: 12 94.0, 24 82.3 us), walls alone 12 (8: 99.8, 16:
 // 88.9).
@@ -311,7 +331,7 @@ int refresh_flat_rules(lbm_lattice* h)
        "rule quad count");
     CK(cudaStreamSynchronize(h->stream), "rule quad sync");
     const long long rules = h->rule_counts[0], plain = quads > rules ? quads - rules : 1;
-    h->flat_on = h->n >= 200000 + 6 * 200000 * rules / quads;
+    h->flat_on = h->flat_set < 0 ? h->n >= flat_min_cells(h, (double)rules / quads) : h->flat_set != 0;
     const long long share = h->has_flags ? 16 : 12;
     const long long want = rules * share * h->sms / plain + 1;
     h->rules_grid = rules > 0 ? (int)(want > 4 * h->sms ? 4 * h->sms : want) : 0;
@@ -1045,6 +1065,19 @@ int lbm_get_rule_blocks(const lbm_lattice* h, int32_t* blocks, int32_t* rule_qua
 }
 
 int64_t lbm_step_count(const lbm_lattice* h) { return h ? h->steps : -1; }
+
+int lbm_test_flat_quads(lbm_lattice* h, int32_t mode, int32_t* in_use)
+{
+    int rc = check_handle(h);
+    if (rc) return rc;
+    if (mode < -1 || mode > 1) return fail(LBM_ERR_INVALID, "mode must be -1, 0 or 1");
+    if (mode == 1 && !h->flat4) return fail(LBM_ERR_UNSUPPORTED, "the lattice cannot step in flat quads");
+    if ((rc = check_no_open_step(h))) return rc;
+    h->flat_set = mode;
+    if (h->flat4 && (rc = refresh_flat_rules(h))) return rc;
+    if (in_use) *in_use = h->flat4 && h->flat_on ? 1 : 0;
+    return LBM_OK;
+}
 
 int lbm_test_barrier_limit(lbm_lattice* h, int32_t missing_arrivals, int64_t timeout_ns)
 {

@@ -66,6 +66,7 @@ struct lbm_lattice {
     // for (refresh_flat_rules).  vec is that of the other steps.
     bool flat4 = false;
     bool flat_on = false;
+    int flat_set = -1;          // lbm_test_flat_quads (-1: by flat_min_cells)
     int rules_grid = 0;
     int rules_grid_set = 0;     // lbm_set_rule_blocks (0: sized from the lists)
     int sms = 148;              // SMs of the lattice's device

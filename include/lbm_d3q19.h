@@ -364,6 +364,13 @@ int lbm_moment16_step(lbm_lattice* h, const double* lo, const double* hi, int32_
  * invalid until new populations are set.  (0, 0) restores the defaults. */
 int lbm_test_barrier_limit(lbm_lattice* h, int32_t missing_arrivals, int64_t timeout_ns);
 
+/* Test hook of the four-cell steps of f16 / bf16 lattices with an odd nz
+ * (lbm_desc.cells_per_thread 0): mode -1 leaves their use to the lattice's size
+ * (the default), 0 switches them off, 1 on (LBM_ERR_UNSUPPORTED where the
+ * lattice cannot step so).  *in_use (optional): whether steps now use them.
+ * Results do not depend on it. */
+int lbm_test_flat_quads(lbm_lattice* h, int32_t mode, int32_t* in_use);
+
 /* ---- without device allocation ----------------------------------------- */
 /* No counterpart in the reference.  FP64 sums {sum rho, sum m_x, sum m_y,
  * sum m_z} of a population array f (19, nx, ny, nz, f64, device memory) over
