@@ -1025,7 +1025,12 @@ int lbm_step_planes(lbm_lattice* h, int32_t x_begin, int32_t x_end)
     a.rule_quads = h->rule_quads;
     for (int k = 0; k < QUAD_KINDS; ++k) a.rule_counts[k] = h->rule_counts[k];
     a.rules_grid = h->rules_grid;
-    a.flat = h->flat4 && h->flat_on;
+    // The flat quads' leading blocks go through the whole lattice's rule cells in
+    // every launch: thin windows step one cell per thread.  A step as one wide
+    // window and four of a plane, us in flat quads throughout / so / one cell
+    // throughout: f16 256x128x127 channel 114.5 / 98.9 / 111.7, 96x96x95 43.2 / 35.0 /
+    // 35.2.
+    a.flat = h->flat4 && h->flat_on && 2 * (long long)(a.P.cell_end - a.P.cell0) >= h->n;
     cudaError_t e = h->storage == LBM_STORAGE_F64 ? launch_exact(KERNEL_STEP, h->desc.force_mode, a)
                                                   : launch_fast(h->storage, KERNEL_STEP, h->desc.force_mode, a);
     if (e != cudaSuccess) return cuda_fail(e, "plane-range step launch");

@@ -90,3 +90,29 @@ def test_bits_of_the_one_cell_kernel(storage):
                 got.append((lat.get_populations(), *lat.rho_u()))
         for a, b in zip(*got, strict=True):
             assert a.tobytes() == b.tobytes(), (shape, force, periodic, flags is not None)
+
+
+def test_windows_of_planes():
+    """Windows of any width (wide ones in flat quads, thin ones one cell per thread), in any
+    order, give the bits of whole steps."""
+    shape = (24, 11, 7)
+    flags = (np.random.default_rng(2).random(shape) < 0.05).astype(np.uint8)
+    f0 = random_state(shape, 12, amp=0.02)
+    for windows in ([(0, 24)], [(0, 12), (12, 24)], [(1, 23), (0, 1), (23, 24)], [(0, 13), (13, 24)],
+                    [(x, x + 1) for x in range(24)]):
+        got = []
+        for mode in (0, 1):
+            with Lattice(shape, 0.65, storage="f16", periodic=Y, wall_velocity=WALLS) as lat:
+                lat.set_flags(flags)
+                _flat(lat, mode)
+                lat.set_populations(f0)
+                lat.step(1)
+                for _ in range(4):
+                    if mode == 0:
+                        lat.step(1)
+                        continue
+                    for w in windows:
+                        lat.step_planes(*w)
+                    lat.step_commit()
+                got.append(lat.get_populations())
+        assert got[0].tobytes() == got[1].tobytes(), windows
