@@ -1666,8 +1666,10 @@ struct lbm_batch {
     bool graph_valid = false;
     // SCHED_BRANCHES: `grid` streams; lattice i steps on branches[branch_of[i]]
     // (largest lattices first, each to the branch with the fewest cells).  A
-    // graph holds every lattice's buffers and parameters: it is recaptured
-    // when a lattice's buffer parity or parameters differ from the capture's.
+    // graph holds every lattice's buffers and parameters: there is one for each
+    // buffer parity (of the first lattice: calls of odd step counts alternate
+    // between them), and it is recaptured when a lattice's own parity or
+    // parameters differ from the capture's.
     std::vector<cudaStream_t> branches;
     std::vector<cudaEvent_t> branch_done;
     cudaEvent_t root = nullptr;
@@ -1676,7 +1678,9 @@ struct lbm_batch {
         cudaGraphExec_t exec = nullptr;
         std::vector<int> cur, params;
     };
-    BranchGraph branch_graph[2];  // of BRANCH_GRAPH_STEPS[k] steps
+    BranchGraph branch_graph[2][2];  // of BRANCH_GRAPH_STEPS[k] steps; by parity
+    int graph_captures = 0;
+    size_t graph_bytes = (size_t)512 << 20;  // BRANCH_GRAPH_STEPS[1] up to this many population bytes
 };
 
 namespace {
@@ -1768,11 +1772,16 @@ int batch_build_branches(lbm_batch* b, int nb)
 // one after the other, each through all the graph's steps, while it sits in
 // L2.  Eight steps against two with a join after each: 16 cavities of up to
 // 96^3 (f16), 20 steps and readbacks, 2.10 -> 1.95 ms.  A batch of many times
-// L2 keeps graphs of two steps with a join after each: 64 cavities, 2.5 GB, on 8
-// branches 38.2 GLUPS so and 36.7 in eights.
+// L2 (graph_bytes) gains nothing from that and keeps graphs of two steps with a
+// join after each, of a quarter of the nodes.  Time of twos over eights, six-wall
+// cavities on 8 branches, f16: 0.35 GB 1.07, 0.6 GB 1.02, 0.8-0.9 GB 1.01, 1.3 GB
+// 1.00-1.02, 2-2.8 GB 0.99-1.00; f32: 1.3 GB 1.00, 2.3-5 GB 1.00-1.01.
+// What a call leaves over eight-step graphs takes two-step graphs and at most
+// one launched step; a graph for each parity spares calls of odd counts the
+// capture.  15 steps, two-step graphs only / rest of eights launched / so: 200
+// lattices of 8-16 cells a side 4.3 / 9.3 / 2.3 ms, 32 of 24-48 1.75 / 2.17 / 0.73.
 constexpr int BRANCH_GRAPH_STEPS[2] = {2, 8};
 constexpr int BRANCH_GRAPH_NODES = 4096;  // more launches than this are not put into one graph
-constexpr size_t BRANCH_GRAPH_BYTES = (size_t)512 << 20;  // nor eight steps of more population bytes
 
 size_t batch_bytes(const lbm_batch* b)
 {
@@ -1826,21 +1835,21 @@ bool branch_graph_current(const lbm_batch* b, const lbm_batch::BranchGraph& g)
 
 void drop_branch_graphs(lbm_batch* b)
 {
-    for (auto& g : b->branch_graph) {
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
-    }
+    for (auto& size : b->branch_graph)
+        for (auto& g : size) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g.exec = nullptr;
+        }
 }
 
-int capture_branch_graph(lbm_batch* b, int which)
+int capture_branch_graph(lbm_batch* b, int which, lbm_batch::BranchGraph& g)
 {
-    auto& g = b->branch_graph[which];
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "graph capture begin");
     cudaError_t e0;
-    if (which == 0 && batch_bytes(b) > BRANCH_GRAPH_BYTES) {
+    if (which == 0 && batch_bytes(b) > b->graph_bytes) {
         e0 = batch_branch_steps(b, 0, 1, false);
         if (e0 == cudaSuccess) e0 = batch_branch_steps(b, 1, 1, false);
     } else {
@@ -1854,6 +1863,7 @@ int capture_branch_graph(lbm_batch* b, int which)
     const cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return cuda_fail(e, "branch graph instantiate");
+    b->graph_captures += 1;
     g.cur.resize(b->count);
     g.params.resize(b->count);
     for (int i = 0; i < b->count; ++i) {
@@ -2018,6 +2028,16 @@ int lbm_batch_get_schedule(const lbm_batch* b, int32_t* sched, int32_t* block, i
     return LBM_OK;
 }
 
+int lbm_test_branch_graphs(lbm_batch* b, int64_t max_bytes, int32_t* captures)
+{
+    if (!b) return fail(LBM_ERR_INVALID, "null batch handle");
+    CK(cudaSetDevice(b->device), "cudaSetDevice");
+    b->graph_bytes = max_bytes >= 0 ? (size_t)max_bytes : (size_t)512 << 20;
+    drop_branch_graphs(b);  // two-step graphs differ on the two sides of the bound
+    if (captures) *captures = b->graph_captures;
+    return LBM_OK;
+}
+
 int lbm_batch_synchronize(lbm_batch* b)
 {
     if (!b) return fail(LBM_ERR_INVALID, "null batch handle");
@@ -2050,16 +2070,21 @@ int lbm_batch_step(lbm_batch* b, int32_t n_steps)
     const int rest = n_steps - done;
     if (rest <= 0) return LBM_OK;
     if (b->sched == SCHED_BRANCHES) {
-        // Whole graphs of eight steps, the rest launched (a call of fewer steps, a
-        // large batch: whole graphs of two).
-        const int which = rest >= BRANCH_GRAPH_STEPS[1] && b->count * BRANCH_GRAPH_STEPS[1] <= BRANCH_GRAPH_NODES &&
-                          batch_bytes(b) <= BRANCH_GRAPH_BYTES;
-        const int per = BRANCH_GRAPH_STEPS[which];
-        if (rest >= per && !branch_graph_current(b, b->branch_graph[which]) && (rc = capture_branch_graph(b, which)))
-            return rc;
-        for (int k = 0; k + per <= rest; k += per)
-            CK(cudaGraphLaunch(b->branch_graph[which].exec, b->stream), "branch graph launch");
-        if (rest % per) CK(batch_branch_steps(b, 0, rest % per, false), "branch step launch");
+        // Whole graphs of eight steps, then of two, then a launched step.  Every
+        // graph is of an even number of steps: the parity is that of the call.
+        auto replay = [&](int which, int times) {
+            if (times == 0) return LBM_OK;
+            auto& g = b->branch_graph[which][b->lats[0]->cur];
+            int r = branch_graph_current(b, g) ? LBM_OK : capture_branch_graph(b, which, g);
+            for (int k = 0; r == LBM_OK && k < times; ++k)
+                if (cudaError_t e = cudaGraphLaunch(g.exec, b->stream)) r = cuda_fail(e, "branch graph launch");
+            return r;
+        };
+        const bool eights =
+            b->count * BRANCH_GRAPH_STEPS[1] <= BRANCH_GRAPH_NODES && batch_bytes(b) <= b->graph_bytes;
+        const int left = eights ? rest % BRANCH_GRAPH_STEPS[1] : rest;
+        if ((rc = replay(1, (rest - left) / BRANCH_GRAPH_STEPS[1])) || (rc = replay(0, left / 2))) return rc;
+        if (left % 2) CK(batch_branch_steps(b, 0, 1, false), "branch step launch");
         batch_advance_bookkeeping(b, rest);
         return LBM_OK;
     }

@@ -126,6 +126,7 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     "lbm_diagnostics": ([_h, C.c_double, _dp], C.c_int),
     "lbm_test_barrier_limit": ([_h, C.c_int32, C.c_int64], C.c_int),
     "lbm_test_flat_quads": ([_h, C.c_int32, C.POINTER(C.c_int32)], C.c_int),
+    "lbm_test_branch_graphs": ([_h, C.c_int64, C.POINTER(C.c_int32)], C.c_int),
     "lbm_moment16_basis": ([_dp, _dp], C.c_int),
     "lbm_moment16_calibrate": ([_h, C.c_int32, C.c_double, _dp, _dp], C.c_int),
     "lbm_moment16_step": ([_h, _dp, _dp, C.c_int32], C.c_int),

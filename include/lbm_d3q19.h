@@ -371,6 +371,11 @@ int lbm_test_barrier_limit(lbm_lattice* h, int32_t missing_arrivals, int64_t tim
  * Results do not depend on it. */
 int lbm_test_flat_quads(lbm_lattice* h, int32_t mode, int32_t* in_use);
 
+/* Test hook of LBM_SCHED_BRANCHES: eight-step graphs are used up to max_bytes
+ * of populations (negative: the default, 512 MB); the captured graphs are
+ * dropped.  *captures (optional): graphs captured since the batch's creation. */
+int lbm_test_branch_graphs(lbm_batch* b, int64_t max_bytes, int32_t* captures);
+
 /* ---- without device allocation ----------------------------------------- */
 /* No counterpart in the reference.  FP64 sums {sum rho, sum m_x, sum m_y,
  * sum m_z} of a population array f (19, nx, ny, nz, f64, device memory) over

@@ -1,0 +1,79 @@
+"""Branch graphs of batches: eight-step and two-step graphs, their remainders,
+both buffer parities, parameter changes between calls, and both sides of the
+size bound, bit for bit against one launch per lattice; and how often graphs
+are captured."""
+
+from __future__ import annotations
+
+import ctypes as C
+
+import pytest
+from gpu_cases import random_state
+from helpers import same_bytes
+
+from lattice_boltzmann_d3q19_b200 import Batch
+from lattice_boltzmann_d3q19_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(9, 8, 7), (12, 6, 10), (5, 11, 16), (16, 9, 3), (7, 7, 12), (6, 30, 9)]
+SIX = (False, False, False)
+
+
+def _specs(storage):
+    return [dict(shape=s, tau=0.55 + 0.05 * k, storage=storage, periodic=SIX if k % 2 else (True, False, True),
+                 wall_velocity={"y+": (0.02 * (k + 1), 0.0, 0.0)}) for k, s in enumerate(SHAPES)]
+
+
+def _captures(b, max_bytes=-1) -> int:
+    n = C.c_int32()
+    N.check(N.lib().lbm_test_branch_graphs(b._h, max_bytes, C.byref(n)))
+    return n.value
+
+
+@pytest.mark.parametrize("storage", ["f64", "f32", "f16"])
+@pytest.mark.parametrize("max_bytes", [-1, 0])  # eight-step graphs; two-step graphs with a join after each step
+def test_counts_and_changes(storage, max_bytes):
+    specs = _specs(storage)
+    with Batch(specs) as a, Batch(specs) as b:
+        a.set_schedule("branches", 128, 3)
+        _captures(a, max_bytes)
+        for k, sp in enumerate(specs):
+            f = random_state(sp["shape"], 80 + k, amp=0.01)
+            a[k].set_populations(f)
+            b[k].set_populations(f)
+        for n in (9, 16, 15, 8, 1, 15, 2, 17, 3, 10):
+            a.step(n)
+            b.step_unbatched(n)
+            for k in range(len(specs)):
+                assert same_bytes(a[k].get_populations(), b[k].get_populations()), (n, k)
+        for x in (a, b):
+            x[2].set_tau(0.65)
+        a.step(15)
+        b.step_unbatched(15)
+        for x in (a, b):
+            x[1].step(1)  # the lattices' parities now differ
+        for n in (8, 9, 24, 7):
+            a.step(n)
+            b.step_unbatched(n)
+        for x in (a, b):
+            x[0].set_wall_velocity("y+", (0.03, 0.0, 0.0))
+        a.step(22)
+        b.step_unbatched(22)
+        for k in range(len(specs)):
+            assert same_bytes(a[k].get_populations(), b[k].get_populations()), k
+            assert a[k].step_count == b[k].step_count
+
+
+@pytest.mark.parametrize("max_bytes,graphs", [(-1, 4), (0, 2)])
+def test_odd_counts_do_not_capture_anew(max_bytes, graphs):
+    with Batch(_specs("f16")) as a:
+        a.set_schedule("branches", 128, 3)
+        before = _captures(a, max_bytes)
+        a.step(1)
+        for _ in range(12):
+            a.step(15)  # 8 + 3 x 2 + 1, from either parity
+            a.step(8)
+        now = C.c_int32()
+        N.check(N.lib().lbm_test_branch_graphs(a._h, max_bytes, C.byref(now)))
+        assert now.value - before == graphs
