@@ -2171,6 +2171,13 @@ int lbm_batch_autotune(lbm_batch* b, int32_t trial_steps, double* best_ms)
                     if (sc == SCHED_BRANCHES && blk != 128) continue;
                     const int g = sc == SCHED_BRANCHES ? 2 * per_sm : per_sm * b->sms;
                     if ((rc = lbm_batch_set_schedule(b, sc, blk, g))) break;
+                    // Branch graphs depend on the step count: those that the timed
+                    // call replays are captured first, and have run before it starts
+                    // (a call's launches are part of its time, a capture is not).
+                    if (sc == SCHED_BRANCHES) {
+                        if ((rc = lbm_batch_step(b, trial_steps))) break;
+                        cudaStreamSynchronize(b->stream);
+                    }
                     if ((rc = lbm_batch_step(b, 2))) break;  // capture + warm
                     cudaEventRecord(e0, b->stream);
                     if ((rc = lbm_batch_step(b, trial_steps))) break;

@@ -6,7 +6,9 @@ are captured."""
 from __future__ import annotations
 
 import ctypes as C
+import time
 
+import numpy as np
 import pytest
 from gpu_cases import random_state
 from helpers import same_bytes
@@ -77,3 +79,26 @@ def test_odd_counts_do_not_capture_anew(max_bytes, graphs):
         now = C.c_int32()
         N.check(N.lib().lbm_test_branch_graphs(a._h, max_bytes, C.byref(now)))
         assert now.value - before == graphs
+
+
+def test_autotune_times_no_capture():
+    """The time that autotune reports is that of the chosen schedule with its graphs captured (a
+    running program's), whatever the trial's step count, and the choice does not depend on it."""
+    rng = np.random.default_rng(3)
+    specs = [dict(shape=tuple(int(v) for v in rng.integers(24, 49, 3)), tau=0.6, storage="f16", periodic=SIX)
+             for _ in range(32)]
+    with Batch(specs) as b:
+        b.step(2)
+        for n in (8, 20):
+            ms = b.autotune(n)
+            b.step(n)
+            times = []
+            for _ in range(20):
+                b.synchronize()
+                t = time.perf_counter()
+                b.step(n)
+                b.synchronize()
+                times.append((time.perf_counter() - t) * 1e3 / n)
+            # 47 us a step, and 13 more while a capture was timed (60 chosen over it)
+            assert ms < 1.12 * min(times), (n, ms, min(times), b.schedule())
+            assert b.schedule()[0] == "branches"
