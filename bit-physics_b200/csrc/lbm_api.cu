@@ -1,7 +1,6 @@
 // lbm_api.cu -- the C ABI of include/lbm_d3q19.h: lattice handles, state
 // transfer, the step loop and the stateless reference functions.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -52,16 +51,6 @@ int cuda_fail(cudaError_t e, const char* what)
         return fail(LBM_ERR_NOMEM, "%s: %s", what, cudaGetErrorString(e));
     }
     return fail(LBM_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-}
-
-cudaError_t device_alloc(void** p, size_t bytes)
-{
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && drop_arenas(0)) {
-        cudaGetLastError();
-        e = cudaMalloc(p, bytes);
-    }
-    return e;
 }
 
 }  // namespace api
@@ -378,7 +367,7 @@ int check_no_open_step(const lbm_lattice* h)
 int ensure_staging(lbm_lattice* h)
 {
     if (h->staging) return LBM_OK;
-    CK(device_alloc((void**)&h->staging, sizeof(double) * Q * (size_t)h->n), "staging allocation");
+    CK(cudaMalloc((void**)&h->staging, sizeof(double) * Q * (size_t)h->n), "staging allocation");
     return LBM_OK;
 }
 
@@ -540,9 +529,7 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     if (desc->device < 0 || desc->device >= ndev) return fail(LBM_ERR_INVALID, "device %d out of range", desc->device);
     CK(cudaSetDevice(desc->device), "cudaSetDevice");
 
-    static std::atomic<uint64_t> next_id{1};
     lbm_lattice* h = new lbm_lattice();
-    h->id = next_id++;
     h->desc = *desc;
     h->storage = desc->storage;
     h->n = desc->nx * desc->ny * desc->nz;
@@ -576,12 +563,12 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     // that may reach past it (the values are not used)
     const size_t pop_bytes = h->state_bytes() + 64;
     for (int b = 0; b < 2; ++b) {
-        e = device_alloc((void**)&h->buf[b], pop_bytes);
+        e = cudaMalloc(&h->buf[b], pop_bytes);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "population allocation"));
     }
     const size_t cbytes = h->storage == LBM_STORAGE_F64 ? sizeof(double) : sizeof(float);
-    e = device_alloc((void**)&h->rho, cbytes * (size_t)h->n);
-    if (e == cudaSuccess) e = device_alloc((void**)&h->u, cbytes * 3 * (size_t)h->n);
+    e = cudaMalloc(&h->rho, cbytes * (size_t)h->n);
+    if (e == cudaSuccess) e = cudaMalloc(&h->u, cbytes * 3 * (size_t)h->n);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "readback allocation"));
     // TMA-staged step (on request): shared-memory pipeline for f32-arithmetic
     // storages whose rows are multiples of 16 bytes.  Not the default: on the
@@ -623,9 +610,9 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     h->partial_blocks = grid_for(h->n, h->block);
     if (h->partial_blocks < h->tma_grid) h->partial_blocks = h->tma_grid;
     if (h->partial_blocks < h->sums_grid) h->partial_blocks = h->sums_grid;
-    e = device_alloc((void**)&h->partials, sizeof(double) * 2 * 5 * (size_t)h->partial_blocks);
-    if (e == cudaSuccess) e = device_alloc((void**)&h->sums, sizeof(double) * 5);
-    if (e == cudaSuccess) e = device_alloc((void**)&h->err, sizeof(int));
+    e = cudaMalloc((void**)&h->partials, sizeof(double) * 2 * 5 * (size_t)h->partial_blocks);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&h->sums, sizeof(double) * 5);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&h->err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "reduction scratch allocation"));
     if (desc->staging == LBM_STAGING_PERSISTENT) {
@@ -634,12 +621,12 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
             cudaGetLastError();
             return cleanup(fail(LBM_ERR_UNSUPPORTED, "persistent staging needs cooperative launch support"));
         }
-        e = device_alloc((void**)&h->bar, sizeof(GridBarrier));
+        e = cudaMalloc((void**)&h->bar, sizeof(GridBarrier));
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "grid barrier allocation"));
         h->persist = true;
     }
     if (h->vec == 4 || h->flat4) {
-        e = device_alloc((void**)&h->rule_quads,
+        e = cudaMalloc((void**)&h->rule_quads,
                          sizeof(int) * (h->flat4 ? flat_rule_ints((h->n + 3) / 4) : rule_quad_ints(h->n / 4)));
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "four-cell step set-up"));
         if (cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, desc->device) != cudaSuccess ||
@@ -649,7 +636,7 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     rebuild_params(h);
     if (int rc2 = refresh_rule_quads(h)) return cleanup(rc2);
     if (visit_order(h).list) {  // fixed by the periodicity, which does not change after creation
-        e = device_alloc((void**)&h->order, sizeof(int) * face_order_ints(h->n / h->vec));
+        e = cudaMalloc((void**)&h->order, sizeof(int) * face_order_ints(h->n / h->vec));
         if (e == cudaSuccess) e = launch_face_order(h->P, h->vec, h->order, h->stream);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "visit order"));
         h->P.order = h->order;
@@ -669,7 +656,6 @@ int lbm_destroy(lbm_lattice* h)
     if (!h) return LBM_OK;
     cudaSetDevice(h->desc.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    drop_arenas(h->id);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     void* ptrs[] = {h->buf[0], h->buf[1], h->flags, h->bbmask, h->force, h->poro, h->rho,
                     h->u, h->partials, h->sums, h->staging, h->monitor, h->err, h->diag, h->rule_quads, h->bar,
@@ -805,10 +791,10 @@ int lbm_set_flags(lbm_lattice* h, const uint8_t* flags)
     }
     if (!h->flags) {
         // whole words: the quad kernels read four flags at a time
-        CK(device_alloc((void**)&h->flags, (size_t)round_up4(h->n)), "flag allocation");
+        CK(cudaMalloc((void**)&h->flags, (size_t)round_up4(h->n)), "flag allocation");
         CK(cudaMemsetAsync(h->flags, 0, (size_t)round_up4(h->n), h->stream), "flag clear");
     }
-    if (!h->bbmask) CK(device_alloc((void**)&h->bbmask, sizeof(uint32_t) * n), "mask allocation");
+    if (!h->bbmask) CK(cudaMalloc((void**)&h->bbmask, sizeof(uint32_t) * n), "mask allocation");
     CK(cudaMemcpyAsync(h->flags, flags, n, cudaMemcpyHostToDevice, h->stream), "flag upload");
     h->has_flags = true;
     rebuild_params(h);
@@ -831,7 +817,7 @@ int lbm_set_force_field(lbm_lattice* h, const double* force)
         return fail(LBM_ERR_STATE, "lattice was not created with LBM_FORCE_FIELD");
     const size_t cnt = 3 * (size_t)h->n;
     if (h->storage == LBM_STORAGE_F64) {
-        if (!h->force) CK(device_alloc((void**)&h->force, sizeof(double) * cnt), "force allocation");
+        if (!h->force) CK(cudaMalloc(&h->force, sizeof(double) * cnt), "force allocation");
         CK(cudaMemcpyAsync(h->force, force, sizeof(double) * cnt, cudaMemcpyHostToDevice, h->stream), "force upload");
         CK(cudaStreamSynchronize(h->stream), "force sync");
     } else {
@@ -839,7 +825,7 @@ int lbm_set_force_field(lbm_lattice* h, const double* force)
         std::vector<float> tmp(3 * fs, 0.0f);
         for (size_t a = 0; a < 3; ++a)
             for (size_t i = 0; i < n; ++i) tmp[a * fs + i] = (float)force[a * n + i];
-        if (!h->force) CK(device_alloc((void**)&h->force, sizeof(float) * tmp.size()), "force allocation");
+        if (!h->force) CK(cudaMalloc(&h->force, sizeof(float) * tmp.size()), "force allocation");
         CK(cudaMemcpyAsync(h->force, tmp.data(), sizeof(float) * tmp.size(), cudaMemcpyHostToDevice, h->stream),
            "force upload");
         CK(cudaStreamSynchronize(h->stream), "force sync");
@@ -860,7 +846,7 @@ int lbm_set_porosity(lbm_lattice* h, const float* alpha)
     for (size_t i = 0; i < n; ++i)
         if (!(alpha[i] >= 0.0f && alpha[i] <= 1.0f))
             return fail(LBM_ERR_INVALID, "porosity at cell %zu is outside [0, 1]", i);
-    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * (size_t)round_up4(h->n)), "porosity allocation");
+    if (!h->poro) CK(cudaMalloc((void**)&h->poro, sizeof(float) * (size_t)round_up4(h->n)), "porosity allocation");
     CK(cudaMemcpyAsync(h->poro, alpha, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream), "porosity upload");
     CK(cudaStreamSynchronize(h->stream), "porosity sync");
     rebuild_params(h);
@@ -1141,7 +1127,7 @@ int lbm_set_porosity_dev(lbm_lattice* h, const float* alpha)
     CK(cudaMemcpyAsync(&flag, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "flag read");
     CK(cudaStreamSynchronize(h->stream), "porosity check sync");
     if (flag) return fail(LBM_ERR_INVALID, "porosity outside [0, 1] (or NaN)");
-    if (!h->poro) CK(device_alloc((void**)&h->poro, sizeof(float) * (size_t)round_up4(h->n)), "porosity allocation");
+    if (!h->poro) CK(cudaMalloc((void**)&h->poro, sizeof(float) * (size_t)round_up4(h->n)), "porosity allocation");
     CK(cudaMemcpyAsync(h->poro, alpha, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream), "porosity copy");
     rebuild_params(h);
     return LBM_OK;
@@ -1163,9 +1149,9 @@ static size_t capture_frames(lbm_lattice* h, size_t total)
     h->frames = nullptr;
     h->frames_raw = nullptr;
     h->frames_cap = 0;
-    cudaError_t e = device_alloc((void**)&h->frames, sizeof(double) * frame * cap);
+    cudaError_t e = cudaMalloc((void**)&h->frames, sizeof(double) * frame * cap);
     if (e == cudaSuccess && h->storage != LBM_STORAGE_F64)
-        e = device_alloc((void**)&h->frames_raw, sizeof(float) * frame * cap);
+        e = cudaMalloc((void**)&h->frames_raw, sizeof(float) * frame * cap);
     if (e != cudaSuccess) {
         cudaGetLastError();
         if (h->frames) cudaFree(h->frames);
@@ -1240,7 +1226,7 @@ int lbm_step_monitor(lbm_lattice* h, int32_t n_steps, double* sums)
         if (h->monitor) CK(cudaFree(h->monitor), "monitor free");
         h->monitor = nullptr;
         h->monitor_cap = 0;
-        CK(device_alloc((void**)&h->monitor, sizeof(double) * 5 * (size_t)n_steps), "monitor allocation");
+        CK(cudaMalloc((void**)&h->monitor, sizeof(double) * 5 * (size_t)n_steps), "monitor allocation");
         h->monitor_cap = n_steps;
     }
     // Step s writes its per-block partials into one of two buffers; block 0 of
@@ -1351,7 +1337,7 @@ int lbm_diagnostics(lbm_lattice* h, double dx_phys, double* out6)
     if (!out6) return fail(LBM_ERR_INVALID, "null output");
     if (!(dx_phys > 0.0)) return fail(LBM_ERR_INVALID, "dx_phys must be > 0");
     if ((rc = check_force_ready(h))) return rc;
-    if (!h->diag) CK(device_alloc((void**)&h->diag, sizeof(double) * (DIAG_SCRATCH + 6)), "diagnostics scratch");
+    if (!h->diag) CK(cudaMalloc((void**)&h->diag, sizeof(double) * (DIAG_SCRATCH + 6)), "diagnostics scratch");
     double* rho = (double*)h->rho;
     double* u = (double*)h->u;
     if (h->storage != LBM_STORAGE_F64) {  // f64, as lbm_get_rho_u hands it out
@@ -1405,7 +1391,7 @@ int workspace(size_t doubles, double** out)
         g_ws.cap = 0;
     }
     if (!g_ws.ptr) {
-        CK(device_alloc((void**)&g_ws.ptr, sizeof(double) * doubles), "workspace allocation");
+        CK(cudaMalloc((void**)&g_ws.ptr, sizeof(double) * doubles), "workspace allocation");
         g_ws.cap = doubles;
         g_ws.device = dev;
     }
@@ -1454,7 +1440,6 @@ extern "C" {
 
 int lbm_release_workspace(void)
 {
-    drop_arenas(0);
     std::lock_guard<std::mutex> lk(g_ws.mu);
     if (g_ws.ptr) cudaFree(g_ws.ptr);
     g_ws.ptr = nullptr;
@@ -1708,7 +1693,7 @@ int batch_build_items(lbm_batch* b)
         if (b->items) CK(cudaFree(b->items), "batch items free");
         b->items = nullptr;
         b->items_cap = 0;
-        CK(device_alloc((void**)&b->items, sizeof(BatchItem) * items.size()), "batch items allocation");
+        CK(cudaMalloc((void**)&b->items, sizeof(BatchItem) * items.size()), "batch items allocation");
         b->items_cap = (int)items.size();
     }
     CK(cudaMemcpy(b->items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice), "items upload");
@@ -1961,7 +1946,7 @@ int lbm_batch_create(const lbm_desc* descs, int32_t count, lbm_batch** out)
     for (lbm_lattice* h : b->lats)
         if ((rc = lbm_set_stream(h, b->stream))) return cleanup(rc);
     b->host_records.resize(count);
-    e = device_alloc((void**)&b->records, sizeof(BatchLattice<float>) * count);
+    e = cudaMalloc(&b->records, sizeof(BatchLattice<float>) * count);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "batch records"));
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
     if (b->sms < 1) b->sms = 1;
@@ -2133,7 +2118,7 @@ int lbm_batch_autotune(lbm_batch* b, int32_t trial_steps, double* best_ms)
         const size_t bytes = h->state_bytes();
         for (int k = 0; k < 2; ++k) {
             void* p = nullptr;
-            cudaError_t e = device_alloc((void**)&p, bytes);
+            cudaError_t e = cudaMalloc(&p, bytes);
             if (e != cudaSuccess) {
                 for (void* q : saved) cudaFree(q);
                 return cuda_fail(e, "autotune snapshot");

@@ -79,7 +79,6 @@ struct lbm_lattice {
     unsigned persist_missing = 0;
     lbm::TileCfg tile{};
     lbm::Params P{};
-    uint64_t id = 0;  // unique in the process: owner of a kept tape arena
 };
 
 namespace lbm {
@@ -89,12 +88,6 @@ namespace api {
 int fail(int code, const char* fmt, ...);
 // LBM_ERR_NOMEM for allocation failures, LBM_ERR_CUDA otherwise.
 int cuda_fail(cudaError_t e, const char* what);
-
-// cudaMalloc; when memory has run out, the kept tape arenas are freed and the
-// allocation is tried once more.
-cudaError_t device_alloc(void** p, size_t bytes);
-// Kept tape arenas (lbm_tape.cu): free those of one lattice (0: all).
-bool drop_arenas(uint64_t owner);
 
 int check_handle(const lbm_lattice* h);
 // LBM_ERR_STATE when the force model's field has not been set.

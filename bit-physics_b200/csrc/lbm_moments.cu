@@ -241,7 +241,7 @@ int lbm_moment16_calibrate(lbm_lattice* h, int32_t n_steps, double margin, doubl
     if (h->storage != LBM_STORAGE_F64 && h->storage != LBM_STORAGE_F32)
         return fail(LBM_ERR_UNSUPPORTED, "calibration runs on an f64 or f32 lattice");
     double* part = nullptr;
-    CK(device_alloc((void**)&part, sizeof(double) * 2 * Q * ENV_GRID), "envelope scratch");
+    CK(cudaMalloc((void**)&part, sizeof(double) * 2 * Q * ENV_GRID), "envelope scratch");
     std::vector<double> host((size_t)2 * Q * ENV_GRID);
     for (int k = 0; k < Q; ++k) {
         lo[k] = 1e300;
@@ -291,7 +291,7 @@ int lbm_moment16_step(lbm_lattice* h, const double* lo, const double* hi, int32_
     if (n_steps == 0) return LBM_OK;
     MomentCodec C;
     if ((rc = codec_from_ranges(lo, hi, C))) return rc;
-    if (!h->me_codes) CK(device_alloc((void**)&h->me_codes, sizeof(uint16_t) * Q * (size_t)h->n), "code allocation");
+    if (!h->me_codes) CK(cudaMalloc((void**)&h->me_codes, sizeof(uint16_t) * Q * (size_t)h->n), "code allocation");
     const int n = h->n;
     const int grid = grid_for(n, 256);
     int32_t s = 0;

@@ -5,9 +5,8 @@
 //
 // State s_k = the lattice buffer after k steps: s_0 = f_0 (PRE), s_k = P_{k-1}.
 // Memory: ceil(N / K) checkpoints + the final state + K - 1 segment states
-// + two adjoint fields + the special-cell list, all in one device allocation.
-#include <mutex>
-#include <set>
+// + two adjoint fields + the special-cell list, all in one piece: an allocation
+// of the tape's own or the caller's (lbm_tape_forward_in).
 #include <vector>
 
 #include "lbm_adjoint.cuh"
@@ -16,100 +15,13 @@
 using namespace lbm;
 using namespace lbm::api;
 
-namespace {
-
-// A destroyed tape leaves its arena with its lattice, and the lattice's next
-// tape takes it when it fits: an optimisation loop runs one tape an iteration
-// on one lattice, and cudaMalloc + cudaFree of the 5 GB of a 128^3 lattice's
-// 100 steps (checkpoints every 25) took 7.2 of the iteration's 30 ms.  At
-// most one arena per lattice and a sixteenth of the GPU's memory in all are
-// kept; destroying the lattice, lbm_release_workspace or any allocation of
-// this library that finds no memory frees them.  No synchronisation is
-// needed: the next tape of the lattice is enqueued on the same stream behind
-// the last use (lbm_set_stream waits for the old stream).
-struct KeptArena {
-    uint64_t owner;
-    int device;
-    void* p;
-    size_t bytes;
-};
-std::mutex g_arena_mu;
-std::vector<KeptArena> g_kept;
-std::set<uint64_t> g_owners;  // lattices that have taped and still exist
-
-size_t kept_limit()
-{
-    static const size_t limit = [] {
-        size_t free_bytes = 0, total = 0;
-        return cudaMemGetInfo(&free_bytes, &total) == cudaSuccess ? total / 16 : (size_t)0;
-    }();
-    return limit;
-}
-
-// The kept arena of the owner when it holds `need` bytes and at most twice
-// that (a smaller or much larger one is freed).
-void* take_arena(uint64_t owner, size_t need, size_t* bytes)
-{
-    std::lock_guard<std::mutex> lk(g_arena_mu);
-    g_owners.insert(owner);
-    for (size_t i = 0; i < g_kept.size(); ++i) {
-        if (g_kept[i].owner != owner) continue;
-        const KeptArena a = g_kept[i];
-        g_kept.erase(g_kept.begin() + i);
-        if (a.bytes >= need && a.bytes <= 2 * need) {
-            *bytes = a.bytes;
-            return a.p;
-        }
-        cudaFree(a.p);
-        break;
-    }
-    return nullptr;
-}
-
-// Keep an arena for its lattice; false: the caller frees it.
-bool keep_arena(const KeptArena& a)
-{
-    std::lock_guard<std::mutex> lk(g_arena_mu);
-    if (!g_owners.count(a.owner)) return false;  // the lattice is gone
-    size_t held = a.bytes;
-    for (const KeptArena& k : g_kept) {
-        if (k.owner == a.owner) return false;
-        held += k.bytes;
-    }
-    if (held > kept_limit()) return false;
-    g_kept.push_back(a);
-    return true;
-}
-
-}  // namespace
-
-bool lbm::api::drop_arenas(uint64_t owner)
-{
-    std::lock_guard<std::mutex> lk(g_arena_mu);
-    int before = 0;
-    bool any = false;
-    if (cudaGetDevice(&before) != cudaSuccess) return false;
-    for (size_t i = g_kept.size(); i-- > 0;) {
-        if (owner && g_kept[i].owner != owner) continue;
-        cudaSetDevice(g_kept[i].device);
-        cudaFree(g_kept[i].p);
-        g_kept.erase(g_kept.begin() + i);
-        any = true;
-    }
-    cudaSetDevice(before);
-    if (owner) g_owners.erase(owner);
-    return any;
-}
-
 struct lbm_tape {
     lbm_lattice* h = nullptr;
-    uint64_t owner = 0;           // the lattice's id
     int device = 0;
     int32_t n_steps = 0;
     int32_t every = 0;
     int params_version = 0;
-    void* arena = nullptr;
-    size_t arena_bytes = 0;
+    void* arena = nullptr;        // the tape's own allocation (null: the caller's memory)
     int64_t bytes = 0;
     size_t state_bytes = 0;       // exact size of one state
     std::vector<void*> ck;        // s_0, s_K, s_2K, ...
@@ -122,6 +34,7 @@ struct lbm_tape {
     // joined back into the lattice's stream, beside the plain-cell kernel.
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    bool forked = false;  // work of `side` is not joined back (a launch failed)
 };
 
 namespace {
@@ -132,7 +45,8 @@ void free_tape(lbm_tape* t)
 {
     if (!t) return;
     cudaSetDevice(t->device);
-    if (t->arena && !keep_arena({t->owner, t->device, t->arena, t->arena_bytes})) cudaFree(t->arena);
+    if (t->forked) cudaStreamSynchronize(t->side);  // it still works on the tape's memory
+    if (t->arena) cudaFree(t->arena);
     if (t->fork) cudaEventDestroy(t->fork);
     if (t->join) cudaEventDestroy(t->join);
     if (t->side) cudaStreamDestroy(t->side);
@@ -145,6 +59,7 @@ int level(lbm_tape* t, int kind, AdjointArgs& a)
     if (fork) {
         CK(cudaEventRecord(t->fork, a.stream), "fork record");
         CK(cudaStreamWaitEvent(t->side, t->fork, 0), "fork wait");
+        t->forked = true;
     }
     a.special_stream = fork ? t->side : nullptr;
     cudaError_t e = launch_adjoint_level(t->h->storage, t->h->desc.force_mode, kind, a);
@@ -152,7 +67,31 @@ int level(lbm_tape* t, int kind, AdjointArgs& a)
     if (fork) {
         CK(cudaEventRecord(t->join, t->side), "join record");
         CK(cudaStreamWaitEvent(a.stream, t->join, 0), "join wait");
+        t->forked = false;
     }
+    return LBM_OK;
+}
+
+// Sizes of a tape's parts, each a multiple of 256 bytes.
+struct TapeLayout {
+    int32_t every;  // steps per segment
+    int nck;        // checkpoints
+    size_t state, lambda, list, total;
+    TapeLayout(const lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every)
+    {
+        every = checkpoint_every < n_steps ? checkpoint_every : n_steps;
+        nck = (n_steps + every - 1) / every;
+        state = round_up(h->state_bytes(), 256);
+        lambda = round_up(adjoint_elem_bytes(h->storage) * Q * (size_t)h->n, 256);
+        list = round_up(sizeof(int) * special_list_ints(h->n), 256);
+        total = ((size_t)nck + 1 + (size_t)(every - 1)) * state + 2 * lambda + list;
+    }
+};
+
+int check_tape_steps(int32_t n_steps, int32_t checkpoint_every)
+{
+    if (n_steps < 1) return fail(LBM_ERR_INVALID, "a tape needs at least one step (got %d)", n_steps);
+    if (checkpoint_every < 1) return fail(LBM_ERR_INVALID, "checkpoint_every must be >= 1");
     return LBM_OK;
 }
 
@@ -162,21 +101,38 @@ extern "C" {
 
 int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, lbm_tape** out)
 {
+    return lbm_tape_forward_in(h, n_steps, checkpoint_every, nullptr, 0, out);
+}
+
+int64_t lbm_tape_need(const lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every)
+{
+    if (!h) return fail(LBM_ERR_INVALID, "null lattice handle");
+    if (int rc = check_tape_steps(n_steps, checkpoint_every)) return rc;
+    return (int64_t)TapeLayout(h, n_steps, checkpoint_every).total;
+}
+
+int lbm_tape_forward_in(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, void* memory, int64_t bytes,
+                        lbm_tape** out)
+{
     if (!out) return fail(LBM_ERR_INVALID, "null output pointer");
     *out = nullptr;
     int rc = check_handle(h);
     if (rc) return rc;
     if ((rc = check_force_ready(h))) return rc;
-    if (n_steps < 1) return fail(LBM_ERR_INVALID, "a tape needs at least one step (got %d)", n_steps);
-    if (checkpoint_every < 1) return fail(LBM_ERR_INVALID, "checkpoint_every must be >= 1");
+    if ((rc = check_tape_steps(n_steps, checkpoint_every))) return rc;
     if (!h->pre)
         return fail(LBM_ERR_STATE, "a tape starts from populations set by lbm_set_populations / "
                                    "lbm_set_equilibrium and not stepped since");
-    const int32_t every = checkpoint_every < n_steps ? checkpoint_every : n_steps;
-    const int nck = (n_steps + every - 1) / every;
+    const TapeLayout L(h, n_steps, checkpoint_every);
+    const int32_t every = L.every;
+    const int nck = L.nck;
+    if (memory) {
+        if ((rc = check_device_ptr(h, memory, "tape memory"))) return rc;
+        if (bytes < 0 || (size_t)bytes < L.total || (uintptr_t)memory % 256 != 0)
+            return fail(LBM_ERR_INVALID, "tape memory must be %zu bytes, 256-byte aligned", L.total);
+    }
     lbm_tape* t = new lbm_tape();
     t->h = h;
-    t->owner = h->id;
     t->device = h->desc.device;
     t->n_steps = n_steps;
     t->every = every;
@@ -188,17 +144,8 @@ int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, 
         free_tape(t);
         return cuda_fail(es, "tape stream / event creation");
     }
-    const size_t sb = round_up(t->state_bytes, 256);
-    const size_t lb = round_up(adjoint_elem_bytes(h->storage) * Q * (size_t)h->n, 256);
-    const size_t nstates = (size_t)nck + 1 + (size_t)(every - 1);
-    const size_t listb = round_up(sizeof(int) * special_list_ints(h->n), 256);
-    const size_t total = nstates * sb + 2 * lb + listb;
-    cudaError_t e = cudaSuccess;
-    t->arena = take_arena(h->id, total, &t->arena_bytes);
-    if (!t->arena) {
-        e = device_alloc(&t->arena, total);
-        t->arena_bytes = total;
-    }
+    const size_t sb = L.state, lb = L.lambda, total = L.total;
+    cudaError_t e = memory ? cudaSuccess : cudaMalloc(&t->arena, total);
     if (e != cudaSuccess) {
         cudaGetLastError();
         free_tape(t);
@@ -207,7 +154,7 @@ int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, 
                     every - 1, cudaGetErrorString(e));
     }
     t->bytes = (int64_t)total;
-    char* p = (char*)t->arena;
+    char* p = (char*)(memory ? memory : t->arena);
     for (int j = 0; j < nck; ++j, p += sb) t->ck.push_back(p);
     t->final_state = p;
     p += sb;

@@ -8,6 +8,7 @@ into it without a CUDA device, raises.
 from __future__ import annotations
 
 import ctypes as C
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -132,6 +133,8 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     "lbm_moment16_step": ([_h, _dp, _dp, C.c_int32], C.c_int),
     "lbm_set_porosity_dev": ([_h, _h], C.c_int),
     "lbm_tape_forward": ([_h, _i, _i, C.POINTER(_h)], C.c_int),
+    "lbm_tape_forward_in": ([_h, _i, _i, _h, C.c_int64, C.POINTER(_h)], C.c_int),
+    "lbm_tape_need": ([_h, _i, _i], C.c_int64),
     "lbm_tape_backward": ([_h, _h, _h, _h, _h], C.c_int),
     "lbm_tape_bytes": ([_h], C.c_int64),
     "lbm_tape_destroy": ([_h], C.c_int),
@@ -141,7 +144,34 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     "lbm_release_workspace": ([], C.c_int),
 }
 
+#: Calls that allocate device memory, before they change anything.
+ALLOCATING = (
+    "lbm_create", "lbm_set_populations", "lbm_get_populations", "lbm_set_equilibrium", "lbm_set_flags",
+    "lbm_set_force_field", "lbm_set_porosity", "lbm_set_porosity_dev", "lbm_step_monitor", "lbm_diagnostics",
+    "lbm_moment16_calibrate", "lbm_moment16_step", "lbm_tape_forward", "lbm_batch_create", "lbm_batch_set_schedule",
+    "lbm_batch_autotune", "lbm_feq_field", "lbm_density_field", "lbm_momentum_field", "lbm_macroscopic_velocity",
+    "lbm_stream", "lbm_bgk_step", "lbm_bounce_back_y_walls",
+)
+
 _lib: C.CDLL | None = None
+
+
+def _again_without_torch_cache(fn):
+    """fn, called a second time where it found no device memory and PyTorch
+    could give back blocks that it only caches (tapes of ``autograd.run``
+    leave theirs there)."""
+
+    def call(*args):
+        rc = fn(*args)
+        if rc == LBM_ERR_NOMEM:
+            torch = sys.modules.get("torch")
+            if torch is not None and torch.cuda.is_initialized():
+                torch.cuda.empty_cache()
+                rc = fn(*args)
+        return rc
+
+    call.argtypes, call.restype = fn.argtypes, fn.restype
+    return call
 
 
 def lib() -> C.CDLL:
@@ -158,6 +188,8 @@ def lib() -> C.CDLL:
             fn = getattr(lib_, name)
             fn.argtypes = args
             fn.restype = res
+        for name in ALLOCATING:
+            setattr(lib_, name, _again_without_torch_cache(getattr(lib_, name)))
         _lib = lib_
     return _lib
 

@@ -30,6 +30,20 @@ def _bind(lattice: Lattice) -> bool:
     return True
 
 
+def _tape_memory(lattice: Lattice, n_steps: int, checkpoint_every: int) -> torch.Tensor | None:
+    """The tape's memory, from PyTorch's allocator: an optimisation loop runs
+    one tape an iteration, and cudaMalloc + cudaFree of the 5 GB of a 128^3
+    lattice's 100 steps (checkpoints every 25) take 4-7 of its 30 ms.  Left in
+    PyTorch's cache between iterations, it serves the program's other tensors
+    too.  Allocated on the current stream, on which the lattice runs (_bind).
+    None where PyTorch has no room: the engine then tries for itself."""
+    try:
+        return torch.empty(lattice.tape_bytes(n_steps, checkpoint_every), dtype=torch.uint8,
+                           device=torch.device("cuda", lattice.desc.device))
+    except torch.OutOfMemoryError:
+        return None
+
+
 class _LatticeRun(torch.autograd.Function):
     @staticmethod
     def forward(ctx, alpha, f0, lattice: Lattice, n_steps: int, checkpoint_every: int):
@@ -46,12 +60,15 @@ class _LatticeRun(torch.autograd.Function):
             lattice.set_equilibrium()
         else:
             lattice.set_populations(f0.detach().to("cpu", torch.float64).numpy())
-        tape = lattice.tape(n_steps, checkpoint_every)
-        rho = torch.empty(shape, dtype=torch.float64, device="cuda")
-        u = torch.empty((3, *shape), dtype=torch.float64, device="cuda")
-        lattice.rho_u_device(rho.data_ptr(), u.data_ptr())
-        if host_sync:
-            lattice.synchronize()
+        memory = _tape_memory(lattice, n_steps, checkpoint_every)
+        try:
+            tape = lattice.tape(n_steps, checkpoint_every, memory)
+            rho = torch.empty(shape, dtype=torch.float64, device="cuda")
+            u = torch.empty((3, *shape), dtype=torch.float64, device="cuda")
+            lattice.rho_u_device(rho.data_ptr(), u.data_ptr())
+        finally:
+            if host_sync:  # also before a failed tape's memory goes back
+                lattice.synchronize()
         ctx.tape = tape
         ctx.alpha_meta = None if alpha is None else (alpha.dtype, alpha.device)
         ctx.f0_meta = None if f0 is None else (f0.dtype, f0.device)
@@ -69,9 +86,13 @@ class _LatticeRun(torch.autograd.Function):
         ga = torch.empty(shape, dtype=torch.float64, device="cuda") if need_alpha else None
         gf = torch.empty((19, *shape), dtype=torch.float64, device="cuda") if need_f0 else None
         host_sync = _bind(lattice)  # after the seeds are ready
-        tape.backward(*(None if t is None else t.data_ptr() for t in (gr, gu, ga, gf)))
-        if host_sync:
-            lattice.synchronize()
+        if tape.memory is not None and not host_sync:
+            tape.memory.record_stream(torch.cuda.current_stream())  # where it differs from forward's
+        try:
+            tape.backward(*(None if t is None else t.data_ptr() for t in (gr, gu, ga, gf)))
+        finally:
+            if host_sync:
+                lattice.synchronize()
         if ga is not None:
             ga = ga.to(dtype=ctx.alpha_meta[0], device=ctx.alpha_meta[1])
         if gf is not None:

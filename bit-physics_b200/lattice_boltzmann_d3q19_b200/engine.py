@@ -332,21 +332,38 @@ class Lattice:
         """set_porosity from n float32 values at a device address."""
         N.check(N.lib().lbm_set_porosity_dev(self._h, C.c_void_p(alpha_ptr)))
 
-    def tape(self, n_steps: int, checkpoint_every: int = 50) -> Tape:
+    def tape(self, n_steps: int, checkpoint_every: int = 50, memory=None) -> Tape:
         """Run n_steps from the current (just set) populations, keeping the
-        checkpoints a backward pass needs; see ``Tape``."""
+        checkpoints a backward pass needs; see ``Tape``.  memory: a CUDA
+        tensor of at least ``tape_bytes(...)`` bytes that the tape holds on to
+        and works in; by default it allocates (and frees) its own."""
         t = C.c_void_p()
-        N.check(N.lib().lbm_tape_forward(self._h, int(n_steps), int(checkpoint_every), C.byref(t)))
-        return Tape(self, t, int(n_steps), int(checkpoint_every))
+        if memory is None:
+            rc = N.lib().lbm_tape_forward(self._h, int(n_steps), int(checkpoint_every), C.byref(t))
+        else:
+            if not memory.is_contiguous():
+                raise ValueError("tape memory must be contiguous")
+            rc = N.lib().lbm_tape_forward_in(self._h, int(n_steps), int(checkpoint_every), memory.data_ptr(),
+                                             memory.numel() * memory.element_size(), C.byref(t))
+        N.check(rc)
+        return Tape(self, t, int(n_steps), int(checkpoint_every), memory)
+
+    def tape_bytes(self, n_steps: int, checkpoint_every: int = 50) -> int:
+        """Device bytes that ``tape(n_steps, checkpoint_every)`` needs."""
+        need = N.lib().lbm_tape_need(self._h, int(n_steps), int(checkpoint_every))
+        if need < 0:
+            N.check(need)
+        return int(need)
 
 
 class Tape:
     """Checkpoints of a forward run (``Lattice.tape``) and the adjoint pass
     back through it.  Pointers are device addresses (integers)."""
 
-    def __init__(self, lattice: Lattice, handle: C.c_void_p, n_steps: int, checkpoint_every: int):
+    def __init__(self, lattice: Lattice, handle: C.c_void_p, n_steps: int, checkpoint_every: int, memory=None):
         self.lattice = lattice  # the tape borrows the lattice: keep it alive
         self._t = handle
+        self.memory = memory
         self.n_steps = n_steps
         self.checkpoint_every = checkpoint_every
 
@@ -369,6 +386,7 @@ class Tape:
         if self._t:
             N.lib().lbm_tape_destroy(self._t)
             self._t = C.c_void_p()
+            self.memory = None
 
     def __del__(self):
         try:

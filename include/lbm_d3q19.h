@@ -320,10 +320,17 @@ typedef struct lbm_tape lbm_tape;
 int lbm_tape_forward(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, lbm_tape** out);
 int lbm_tape_backward(lbm_tape* t, const double* grad_rho, const double* grad_u, double* grad_alpha,
                       double* grad_f0);
-/* Device bytes the tape holds (checkpoints, segment states, adjoint fields).
- * A destroyed tape's memory stays with its lattice for the lattice's next tape
- * (at most one per lattice and a sixteenth of the GPU's memory in all) until
- * the lattice is destroyed or lbm_release_workspace is called. */
+/* The same with the tape's memory supplied by the caller: at least
+ * lbm_tape_need(...) bytes of the lattice's GPU, 256-byte aligned, the caller's
+ * again once the tape is destroyed and the lattice's stream has passed its last
+ * use.  A program that runs one tape after another keeps the memory so instead
+ * of paying cudaMalloc and cudaFree each time.  memory NULL: the tape
+ * allocates and frees its own. */
+int lbm_tape_forward_in(lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every, void* memory, int64_t bytes,
+                        lbm_tape** out);
+/* Device bytes of such a tape (negative: an error code). */
+int64_t lbm_tape_need(const lbm_lattice* h, int32_t n_steps, int32_t checkpoint_every);
+/* Device bytes the tape holds (checkpoints, segment states, adjoint fields). */
 int64_t lbm_tape_bytes(const lbm_tape* t);
 int lbm_tape_destroy(lbm_tape* t);
 
@@ -401,9 +408,7 @@ const char* lbm_last_error(void);
 int lbm_version(void);
 /* Number of visible CUDA devices (0 when there is no driver or device). */
 int lbm_device_count(void);
-/* Release the device memory that the library keeps between calls: the
- * workspace of the host-array functions and the arenas that destroyed tapes
- * have left with their lattices. */
+/* Release the device workspace that the host-array functions cache. */
 int lbm_release_workspace(void);
 
 #ifdef __cplusplus
