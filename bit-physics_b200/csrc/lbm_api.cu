@@ -659,7 +659,7 @@ int lbm_destroy(lbm_lattice* h)
     if (h->graph) cudaGraphExecDestroy(h->graph);
     void* ptrs[] = {h->buf[0], h->buf[1], h->flags, h->bbmask, h->force, h->poro, h->rho,
                     h->u, h->partials, h->sums, h->staging, h->monitor, h->err, h->diag, h->rule_quads, h->bar,
-                    h->me_codes, h->order, h->frames, h->frames_raw};
+                    h->me_codes, h->order};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -1133,34 +1133,78 @@ int lbm_set_porosity_dev(lbm_lattice* h, const float* alpha)
     return LBM_OK;
 }
 
-// Room for the frames of a capture: up to 48 MB of them (kept with the lattice),
-// so that they go to the host in a few large copies.  Copied frame by frame, a
-// 64x32x3 lattice spent 55 us a frame, 9 of them stepping: 200 captured steps
-// 12.5 -> 3.5 ms.  0 where fewer than two frames fit (or nothing does): frame by frame.
-static size_t capture_frames(lbm_lattice* h, size_t total)
-{
-    const size_t frame = 4 * (size_t)h->n;  // values
-    size_t cap = ((size_t)48 << 20) / (sizeof(double) * frame);
-    if (cap > total) cap = total;
-    if (cap < 2) return 0;
-    if (h->frames_cap >= cap) return h->frames_cap;
-    if (h->frames) cudaFree(h->frames);
-    if (h->frames_raw) cudaFree(h->frames_raw);
-    h->frames = nullptr;
-    h->frames_raw = nullptr;
-    h->frames_cap = 0;
-    cudaError_t e = cudaMalloc((void**)&h->frames, sizeof(double) * frame * cap);
-    if (e == cudaSuccess && h->storage != LBM_STORAGE_F64)
-        e = cudaMalloc((void**)&h->frames_raw, sizeof(float) * frame * cap);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        if (h->frames) cudaFree(h->frames);
-        h->frames = nullptr;
-        return 0;
+// Memory that one call works in and leaves for the next: one pool for a GPU,
+// which holds on to what one capture needs, serves any lattice, stream and
+// thread, and gives way to allocations that find no other memory (CUDA frees
+// a pool's unused memory before cudaMalloc fails).  Null: none to be had.
+constexpr size_t CAPTURE_BYTES = (size_t)48 << 20;  // of f64 frames
+struct CallPools {
+    std::mutex mu;
+    std::vector<std::pair<int, cudaMemPool_t>> pools;  // by device
+    cudaMemPool_t get(int device)
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        for (const auto& p : pools)
+            if (p.first == device) return p.second;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e == cudaSuccess) {
+            uint64_t keep = CAPTURE_BYTES + CAPTURE_BYTES / 2;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        } else {
+            cudaGetLastError();
+            pool = nullptr;
+        }
+        pools.emplace_back(device, pool);
+        return pool;
     }
-    h->frames_cap = cap;
-    return cap;
-}
+    void trim()
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        for (const auto& p : pools)
+            if (p.second) cudaMemPoolTrimTo(p.second, 0);
+    }
+};
+static CallPools g_call_pools;
+
+// Room for the frames of a capture, up to 48 MB of them, so that they go to the
+// host in a few large copies.  Copied frame by frame, a 64x32x3 lattice spent 55 us
+// a frame, 9 of them stepping: 200 captured steps 12.5 -> 3.5 ms.  cap 0 where
+// fewer than two frames fit (or nothing does): frame by frame.  However the
+// call ends, nothing of it is still being copied then.
+struct CaptureFrames {
+    lbm_lattice* h;
+    size_t cap = 0;         // frames
+    double* f64 = nullptr;  // rho of every frame, then u
+    float* raw = nullptr;   // the same as the kernels write them where that is f32
+    bool copying = false;
+    CaptureFrames(lbm_lattice* lat, size_t total) : h(lat)
+    {
+        const size_t frame = 4 * (size_t)h->n;  // values
+        cap = CAPTURE_BYTES / (sizeof(double) * frame);
+        if (cap > total) cap = total;
+        const size_t bytes = frame * cap * (sizeof(double) + (h->storage == LBM_STORAGE_F64 ? 0 : sizeof(float)));
+        cudaMemPool_t pool = cap < 2 ? nullptr : g_call_pools.get(h->desc.device);
+        if (!pool || cudaMallocFromPoolAsync((void**)&f64, bytes, pool, h->stream) != cudaSuccess) {
+            cudaGetLastError();
+            f64 = nullptr;
+            cap = 0;
+            return;
+        }
+        if (h->storage != LBM_STORAGE_F64) raw = (float*)(f64 + frame * cap);
+    }
+    CaptureFrames(const CaptureFrames&) = delete;
+    CaptureFrames& operator=(const CaptureFrames&) = delete;
+    ~CaptureFrames()
+    {
+        if (copying) cudaStreamSynchronize(h->stream);
+        if (f64) cudaFreeAsync(f64, h->stream);
+    }
+};
 
 int lbm_run_capture(lbm_lattice* h, int32_t n_steps, int32_t every, double* rho_frames, double* u_frames)
 {
@@ -1172,16 +1216,17 @@ int lbm_run_capture(lbm_lattice* h, int32_t n_steps, int32_t every, double* rho_
     if ((rc = check_force_ready(h))) return rc;
     const size_t n = (size_t)h->n;
     const size_t total = (size_t)n_steps / every + 1 + (n_steps % every ? 1 : 0);
-    const size_t cap = capture_frames(h, total);
+    CaptureFrames frames(h, total);
+    const size_t cap = frames.cap;
     size_t done = 0, held = 0;  // frames on the host; in the buffer
     for (int32_t s = 0; s <= n_steps; ++s) {
         const bool need = (s % every == 0) || (s == n_steps);
         void *rho = h->rho, *u = h->u;
         if (cap && need) {
             const size_t elem = h->storage == LBM_STORAGE_F64 ? sizeof(double) : sizeof(float);
-            char* base = h->storage == LBM_STORAGE_F64 ? (char*)h->frames : (char*)h->frames_raw;
+            char* base = frames.raw ? (char*)frames.raw : (char*)frames.f64;
             rho = base + elem * held * n;
-            u = base + elem * (h->frames_cap + 3 * held) * n;
+            u = base + elem * (cap + 3 * held) * n;
         }
         if (s < n_steps) {
             // The step kernel reads back the state it advances from (step s).
@@ -1195,11 +1240,12 @@ int lbm_run_capture(lbm_lattice* h, int32_t n_steps, int32_t every, double* rho_
             if (rc) return rc;
             ++done;
         } else if (++held == cap || s == n_steps) {
-            double *rd = h->frames, *ud = h->frames + h->frames_cap * n;
-            if (h->storage != LBM_STORAGE_F64) {
-                CK(launch_widen(h->frames_raw, rd, held * n, h->stream), "frame widen");
-                CK(launch_widen(h->frames_raw + h->frames_cap * n, ud, held * 3 * n, h->stream), "frame widen");
+            double *rd = frames.f64, *ud = frames.f64 + cap * n;
+            if (frames.raw) {
+                CK(launch_widen(frames.raw, rd, held * n, h->stream), "frame widen");
+                CK(launch_widen(frames.raw + cap * n, ud, held * 3 * n, h->stream), "frame widen");
             }
+            frames.copying = true;
             CK(cudaMemcpyAsync(rho_frames + done * n, rd, sizeof(double) * held * n, cudaMemcpyDeviceToHost, h->stream),
                "frame copy");
             CK(cudaMemcpyAsync(u_frames + done * 3 * n, ud, sizeof(double) * held * 3 * n, cudaMemcpyDeviceToHost,
@@ -1209,6 +1255,7 @@ int lbm_run_capture(lbm_lattice* h, int32_t n_steps, int32_t every, double* rho_
             held = 0;
         }
     }
+    frames.copying = false;
     CK(cudaStreamSynchronize(h->stream), "capture sync");
     return LBM_OK;
 }
@@ -1440,6 +1487,7 @@ extern "C" {
 
 int lbm_release_workspace(void)
 {
+    g_call_pools.trim();
     std::lock_guard<std::mutex> lk(g_ws.mu);
     if (g_ws.ptr) cudaFree(g_ws.ptr);
     g_ws.ptr = nullptr;

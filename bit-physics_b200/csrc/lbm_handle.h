@@ -33,11 +33,6 @@ struct lbm_lattice {
     double* sums = nullptr;  // 5 doubles
     int partial_blocks = 0;  // rows of partials of one launch (one per block, any kernel)
     double* staging = nullptr; // (19, n) f64, allocated on first use
-    // Frames of lbm_run_capture on their way to the host, `frames_cap` of them:
-    // rho then u as f64, and as the kernels write them where that is f32.
-    double* frames = nullptr;
-    float* frames_raw = nullptr;
-    size_t frames_cap = 0;
     double* monitor = nullptr; // (monitor_cap, 5) per-step sums of lbm_step_monitor
     double* diag = nullptr;    // DIAG_SCRATCH + 6 doubles of lbm_diagnostics, allocated on first use
     uint16_t* me_codes = nullptr; // (19, n) 16-bit moment codes of lbm_moment16_step, allocated on first use

@@ -408,7 +408,9 @@ const char* lbm_last_error(void);
 int lbm_version(void);
 /* Number of visible CUDA devices (0 when there is no driver or device). */
 int lbm_device_count(void);
-/* Release the device workspace that the host-array functions cache. */
+/* Release the device memory that the library keeps between calls: the
+ * workspace of the host-array functions and the frame buffer of
+ * lbm_run_capture (up to 72 MB for each GPU). */
 int lbm_release_workspace(void);
 
 #ifdef __cplusplus
