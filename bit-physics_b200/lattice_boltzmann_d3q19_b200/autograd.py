@@ -35,13 +35,22 @@ def _tape_memory(lattice: Lattice, n_steps: int, checkpoint_every: int) -> torch
     one tape an iteration, and cudaMalloc + cudaFree of the 5 GB of a 128^3
     lattice's 100 steps (checkpoints every 25) take 4-7 of its 30 ms.  Left in
     PyTorch's cache between iterations, it serves the program's other tensors
-    too.  Allocated on the current stream, on which the lattice runs (_bind).
-    None where PyTorch has no room: the engine then tries for itself."""
+    too.  Allocated for the default stream and lent to the current one, on
+    which the lattice runs (_bind), so that tapes on any stream share it: in
+    the cache of each stream's own, every new lattice and stream paid for new
+    pages (25 ms).  None where PyTorch has no room: the engine then tries for
+    itself."""
+    device = torch.device("cuda", lattice.desc.device)
+    stream, default = torch.cuda.current_stream(), torch.cuda.default_stream(device)
     try:
-        return torch.empty(lattice.tape_bytes(n_steps, checkpoint_every), dtype=torch.uint8,
-                           device=torch.device("cuda", lattice.desc.device))
+        with torch.cuda.stream(default):
+            memory = torch.empty(lattice.tape_bytes(n_steps, checkpoint_every), dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
         return None
+    if stream != default:
+        stream.wait_stream(default)  # the block's earlier uses
+        memory.record_stream(stream)
+    return memory
 
 
 class _LatticeRun(torch.autograd.Function):
@@ -87,7 +96,7 @@ class _LatticeRun(torch.autograd.Function):
         gf = torch.empty((19, *shape), dtype=torch.float64, device="cuda") if need_f0 else None
         host_sync = _bind(lattice)  # after the seeds are ready
         if tape.memory is not None and not host_sync:
-            tape.memory.record_stream(torch.cuda.current_stream())  # where it differs from forward's
+            tape.memory.record_stream(torch.cuda.current_stream())  # may differ from forward's
         try:
             tape.backward(*(None if t is None else t.data_ptr() for t in (gr, gu, ga, gf)))
         finally:
