@@ -104,14 +104,15 @@ __device__ __forceinline__ void reduce_prev(const Outputs<C>& out)
     __syncthreads();  // the shared reduction array is reused by the caller
 }
 
-template <class M, int FM, int OUT>
+// BESIDE: the cell collides in the same thread, by itself (readback).
+template <class M, int FM, int OUT, bool BESIDE = false>
 __device__ __forceinline__ void emit(const Params& P, const Outputs<typename M::C>& out, int idx, bool solid,
                                      const typename M::C* f, double* cons)
 {
     using C = typename M::C;
     if constexpr ((OUT & OUT_RHO_U) != 0) {
         C r = C(0), u[3] = {C(0), C(0), C(0)};
-        if (!solid) M::template readback<FM>(P, idx, f, r, u);
+        if (!solid) M::template readback<FM, BESIDE>(P, idx, f, r, u);
         out.rho[idx] = r;
         out.u[idx] = u[0];
         out.u[P.n + idx] = u[1];
@@ -167,7 +168,7 @@ __device__ __forceinline__ void step_single(const Params& P, const Streams<typen
     C f[Q];
     gather<M>(P, S, nb, f);
     if (resolve_state<M>(P, S, idx, x, y, z, fl, nb, f)) {
-        emit<M, FM, OUT>(P, out, idx, false, f, cons);
+        emit<M, FM, OUT, true>(P, out, idx, false, f, cons);
         M::template collide<FM>(P, idx, f);
         store_all<M>(P, S, idx, f);
     } else {
@@ -989,7 +990,7 @@ __device__ __forceinline__ void collide_single(const Params& P, const Streams<ty
         emit<M, FM, OUT>(P, out, idx, true, f, cons);
         store_solid<M>(P, S, idx);
     } else {
-        emit<M, FM, OUT>(P, out, idx, false, f, cons);
+        emit<M, FM, OUT, true>(P, out, idx, false, f, cons);
         M::template collide<FM>(P, idx, f);
         store_all<M>(P, S, idx, f);
     }
