@@ -496,7 +496,8 @@ int lbm_desc_init(lbm_desc* d)
     return LBM_OK;
 }
 
-int lbm_create(const lbm_desc* desc, lbm_lattice** out)
+// flat_quads: the lattice may step with k_step4_flat where that applies.
+static int create_lattice(const lbm_desc* desc, bool flat_quads, lbm_lattice** out)
 {
     if (!desc || !out) return fail(LBM_ERR_INVALID, "null argument to lbm_create");
     *out = nullptr;
@@ -534,7 +535,6 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     h->storage = desc->storage;
     h->n = desc->nx * desc->ny * desc->nz;
     h->elem = storage_bytes(desc->storage);
-    h->stride = storage16 ? round_up4(h->n) : h->n;
     // 128-thread blocks: on the 256x128x128 sphere channel f32 39.5 against
     // 38.9 GLUPS with 256, f16 (pipelined) 59.1 against 58.4 (192: 38.7 /
     // 52.4), f64 17.1 against 16.5.
@@ -550,8 +550,15 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
         h->vec = 4;
     else
         h->vec = desc->storage != LBM_STORAGE_F64 && desc->nz % 2 == 0 ? 2 : 1;
-    h->flat4 = storage16 && desc->cells_per_thread == 0 && desc->nz % 2 != 0 && desc->nz >= FLAT_MIN_NZ &&
+    h->flat4 = flat_quads && storage16 && desc->cells_per_thread == 0 && desc->nz % 2 != 0 &&
+               desc->nz >= FLAT_MIN_NZ &&
                (desc->staging == LBM_STAGING_AUTO || desc->staging == LBM_STAGING_REGISTERS);
+    // Flat quads need every direction 8-byte aligned, but where that puts all of
+    // them on 32-byte sectors the other kernels of these lattices suffer (f16
+    // 195x54x119 channel, step with sums: 53.1 us so, 50.8 four cells further;
+    // 195x54x117 52.7 / 49.0; 130x54x119 alone 26.2 / 26.7).
+    h->stride = h->n;
+    if (h->flat4 && h->n % 4 != 0) h->stride = round_up4(h->n) % 16 != 0 ? round_up4(h->n) : round_up4(h->n) + 4;
     auto cleanup = [&](int code) {
         lbm_destroy(h);
         return code;
@@ -650,6 +657,8 @@ int lbm_create(const lbm_desc* desc, lbm_lattice** out)
     *out = h;
     return LBM_OK;
 }
+
+int lbm_create(const lbm_desc* desc, lbm_lattice** out) { return create_lattice(desc, true, out); }
 
 int lbm_destroy(lbm_lattice* h)
 {
@@ -1999,12 +2008,11 @@ int lbm_batch_create(const lbm_desc* descs, int32_t count, lbm_batch** out)
     int rc;
     for (int i = 0; i < count; ++i) {
         lbm_lattice* h = nullptr;
-        if ((rc = lbm_create(&descs[i], &h))) return cleanup(rc);
         // One cell per thread for odd nz (the same bits): beside other
         // lattices' kernels the flat quads' rule blocks hold SMs that those
         // would use.  16 f16 cavities of up to 96^3, 20 steps on 8 branches:
         // 2.10 ms, with flat quads 2.28.
-        h->flat4 = false;
+        if ((rc = create_lattice(&descs[i], false, &h))) return cleanup(rc);
         b->lats.push_back(h);
     }
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);

@@ -136,8 +136,8 @@ struct Params {
     int nx, ny, nz, n, nynz;
     // Elements from one direction of the population array to the next, and
     // from one component of the force field to the next: n, rounded up to a
-    // multiple of 4 for the 16-bit storages' populations and the f32 force
-    // fields, so that every direction starts 8-byte aligned.
+    // multiple of 4 (or 4 more) for the lattices that may step in flat quads
+    // and for the f32 force fields, so that four cells start 8-byte aligned.
     int stride, force_stride;
     FastDiv div_nz, div_ny;
     int periodic;      // bit 0 x, 1 y, 2 z
