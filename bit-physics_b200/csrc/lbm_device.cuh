@@ -402,16 +402,18 @@ __device__ __forceinline__ double div_exact(double x, double y, double rhi, doub
     return __fma_rn(__fma_rn(-q, y, x), rhi, q);
 }
 
-// High words (sign, exponent, 20 mantissa bits) of the positive doubles in
+// High words (sign, exponent, 20 mantissa bits) of the doubles of magnitude
 // [2^-300, 2^100): the range in which div_exact and the sums of the fast
 // collision stay far from underflow and overflow.
 constexpr uint32_t EXACT_LO = 0x2d300000u, EXACT_SPAN = 0x46300000u - 0x2d300000u;
-// 0 .. EXACT_SPAN - 1 for a value in that range, more for any other.
-__device__ __forceinline__ uint32_t exact_range(double v) { return (uint32_t)__double2hiint(v) - EXACT_LO; }
-__device__ __forceinline__ bool exact_range_or_zero(double v)
+// Below 2 EXACT_SPAN for a value in that range, not below for any other
+// (doubled: the sign drops out).
+__device__ __forceinline__ uint32_t exact_range(double v)
 {
-    return v == 0.0 || exact_range(fabs(v)) < EXACT_SPAN;
+    const uint32_t hi = (uint32_t)__double2hiint(v);
+    return hi + hi - 2 * EXACT_LO;
 }
+__device__ __forceinline__ bool exact_range_or_zero(double v) { return v == 0.0 || exact_range(v) < 2 * EXACT_SPAN; }
 
 template <bool CG = false>
 struct ModeExactT {
@@ -452,7 +454,7 @@ struct ModeExactT {
         double ci_dot_uw = (double)cx(d) * uw[0] + (double)cy(d) * uw[1] + (double)cz(d) * uw[2];
         const double x = -2.0 * P.w[d] * rho_w * ci_dot_uw;
         if (x == 0.0) return x;
-        if (exact_range(fabs(x)) < EXACT_SPAN) return div_exact(x, P.cs2, P.cs2_rhi, P.cs2_rlo);
+        if (exact_range(x) < 2 * EXACT_SPAN) return div_exact(x, P.cs2, P.cs2_rhi, P.cs2_rlo);
         return x / P.cs2;
     }
 
@@ -462,11 +464,13 @@ struct ModeExactT {
     // divisions by tau and 3 by rho a cell.  Here every division is four
     // operations (div_exact), opposite directions share c.u and its square,
     // and the products with a zero velocity component are left out.  That is
-    // exact while every population lies in [2^-300, 2^100): then the sums hold
-    // no negative zero that an added +-0 would change, an opposite direction's
-    // terms are exact negations, and no intermediate under- or overflows.  A
-    // cell outside that range (a negative, zero or non-finite population) or
-    // a force outside it takes collide_general.  Measured: 20 steps and a
+    // exact while the magnitude of every population lies in [2^-300, 2^100): then
+    // the sums hold no negative zero that an added +-0 would change (a sum that
+    // cancels is +0), an opposite direction's terms are exact negations, and no
+    // intermediate under- or overflows, also where the density is not positive
+    // and rho_safe puts 1e-30 in its place.  A cell with a zero, tiny, huge or
+    // non-finite population or such a force takes collide_general, a call with
+    // the populations in local memory.  Measured: 20 steps and a
     // readback of the 256x128x128 sphere channel 4.85 -> 4.05 ms (now bound
     // by memory), a step of a 32x16x3 Couette lattice 3.9 -> 2.4 us (latency
     // of one cell's chain of operations).
@@ -476,7 +480,7 @@ struct ModeExactT {
         uint32_t worst = 0;
 #pragma unroll
         for (int d = 0; d < Q; ++d) worst = max(worst, exact_range(f[d]));
-        bool fast = worst < EXACT_SPAN && P.tau_fast;
+        bool fast = worst < 2 * EXACT_SPAN && P.tau_fast;
         double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
 #pragma unroll
         for (int d = 0; d < Q; ++d) {
@@ -559,6 +563,14 @@ struct ModeExactT {
             mx = mx + (double)cx(d) * fd;
             my = my + (double)cy(d) * fd;
             mz = mz + (double)cz(d) * fd;
+        }
+        // A NaN population makes every result NaN: said so without 22 divisions, a
+        // lattice that has blown up steps no slower than before the fast form (all
+        // NaN, us a step, divided inline / here / so: 95x34x176 in six walls 62.7 /
+        // 85.0 / 45.4, 160x128x128 channel with drag 410 / 551 / 180).
+        if (r != r) {
+            for (int d = 0; d < Q; ++d) f[d] = r;
+            return;
         }
         double rs = rho_safe(r);
         double Fx, Fy, Fz;
