@@ -816,7 +816,7 @@ def run_ensemble(args):
         b.step(2)
         dt = timed(lambda: b.step(args.steps))
         out["batched_branches"] = {"glups": cells * args.steps / dt / 1e9, "schedule": list(b.schedule()),
-                                   "launches_per_step": "graphs of per-lattice kernels, eight steps each"}
+                                   "launches_per_step": "graphs of per-lattice kernels, two steps each"}
         ms = b.autotune(20)
         b.step(2)
         dt = timed(lambda: b.step(args.steps))

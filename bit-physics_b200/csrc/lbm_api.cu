@@ -153,8 +153,10 @@ int round_up4(int n) { return (n + 3) / 4 * 4; }
 //               80^3 30.7 / 36.6 / 35.3, 128^3 103 / 158 / 125; f16 128x128x98
 //               57.8 / 45.1 / 42.0
 // Within L2 that is a list, the faces in lattice order (order); tiny f64
-// lattices, a few blocks in all, are left in their rows (32x16x3 with y walls:
-// 2.4 -> 2.1 us).  Beyond, the order is computed (first): a list's load from
+// lattices, a few blocks in all, are left in their rows: list / rows, us a step,
+// y walls 1,536 cells 6.2 / 5.1, 8,000 6.2 / 5.1, six walls 13,824 7.2 / 6.2; at
+// 110,592 cells y walls turn to 6.2 / 7.2.  (Tiny f32 and 16-bit lattices step as
+// fast in rows or faster, 1.00-1.25; they keep the list.)  Beyond, the order is computed (first): a list's load from
 // memory comes before the gather (y walls, f32 128^3: 54.4 -> 52.2 us).  With
 // walls off the z axis it serves f32 and f64 too, unless rows of odd length
 // shift every warp off its cache lines (f32 128x128x127, y walls: 51.5 / 59.5).

@@ -1112,8 +1112,8 @@ __device__ __forceinline__ void read_pair(const Params& P, const Streams<typenam
 // (16-bit storage, nz a multiple of 4: the plain quads' sources are one
 // 8-byte load a direction, as in k_step4).  Bound by memory: populations in,
 // 32 bytes a cell out.  Against k_observe (one cell per thread, f32 fields)
-// and two widening passes, bf16 512x256x256 channel: 1281 -> 539 us; f16 /
-// f32 256x128x128: 172 -> 82, 158 -> 95 us.
+// and two widening passes, bf16 512x256x256 channel: 1311 -> 618 us; f16 /
+// f32 256x128x128: 181 -> 92, 169 -> 109 us.
 template <class M, int FM, int VEC>
 __global__ void __launch_bounds__(128, 4)
     k_read(const __grid_constant__ Params P, const __grid_constant__ Streams<typename M::T> S, bool post, double* rho,

@@ -255,7 +255,8 @@ typedef struct lbm_batch lbm_batch;
 #define LBM_SCHED_BRANCHES 3    /* no batched kernel: every lattice's own step
                                    kernels on `grid` parallel streams (0: 8),
                                    largest lattices first, each to the stream with
-                                   the fewest cells; eight steps per captured graph */
+                                   the fewest cells; captured graphs of eight or
+                                   two steps (lbm_batch_step) */
 
 int lbm_batch_create(const lbm_desc* descs, int32_t count, lbm_batch** out);
 int lbm_batch_destroy(lbm_batch* b);
@@ -269,8 +270,10 @@ int lbm_batch_lattice(lbm_batch* b, int32_t i, lbm_lattice** out);
 int lbm_batch_set_schedule(lbm_batch* b, int32_t sched, int32_t block, int32_t grid);
 int lbm_batch_get_schedule(const lbm_batch* b, int32_t* sched, int32_t* block, int32_t* grid);
 /* Advance every lattice n_steps: one launch per step (LBM_SCHED_BRANCHES:
- * graphs of per-lattice launches, eight steps each), steady-state steps
- * replayed from a captured CUDA graph. */
+ * graphs of per-lattice launches), steady-state steps replayed from captured
+ * CUDA graphs.  Branch graphs hold eight steps; two in calls of fewer, for
+ * what a call leaves over eights, and for batches of more than 512 MB of
+ * populations or 512 lattices. */
 int lbm_batch_step(lbm_batch* b, int32_t n_steps);
 /* The same with one launch per lattice and step (for comparison). */
 int lbm_batch_step_unbatched(lbm_batch* b, int32_t n_steps);
