@@ -156,8 +156,8 @@ int round_up4(int n) { return (n + 3) / 4 * 4; }
 // lattices, a few blocks in all, are left in their rows: list / rows, us a step,
 // y walls 1,536 cells 6.2 / 5.1, 8,000 6.2 / 5.1, six walls 13,824 7.2 / 6.2; at
 // 110,592 cells y walls turn to 6.2 / 7.2.  (Tiny f32 and 16-bit lattices step as
-// fast in rows or faster, 1.00-1.25; they keep the list.)  Beyond, the order is computed (first): a list's load from
-// memory comes before the gather (y walls, f32 128^3: 54.4 -> 52.2 us).  With
+// fast in rows or faster, 1.00-1.25; they keep the list.)  Beyond, the order is
+// computed (first): a list's load from memory comes before the gather (y walls, f32 128^3: 54.4 -> 52.2 us).  With
 // walls off the z axis it serves f32 and f64 too, unless rows of odd length
 // shift every warp off its cache lines (f32 128x128x127, y walls: 51.5 / 59.5).
 struct VisitOrder {
@@ -286,8 +286,8 @@ namespace {
 // quads that need a rule.  A lattice of less than a wave of quads has too few
 // threads to hide its loads, and the cells of rule quads cost more than one by
 // one in their own kernel: on walled faces (moving-wall products on a chain of
-// loads) a lot, off them (flags alone) little.  Flat quads against one cell per
-// thread, time ratio by cells, f16 without force:
+// loads) a lot, off them (flags alone) little.  Time of one cell per thread over
+// that of flat quads by cells, f16 without force:
 //   periodic, r < 0.01       0.25 M 1.00, 0.35 M 1.00-1.12, 0.5 M 1.00-1.08, 1 M
 //                            1.06-1.17, 2 M 1.20, 4 M 1.24 (drag 1.44)
 //   spheres, r 0.02-0.07     0.15 M 0.97-1.09, 0.25 M 1.02-1.19, 0.5 M 1.08-1.18,
@@ -309,8 +309,8 @@ double flat_min_cells(const lbm_lattice* h, double r)
     return h->has_flags ? 200000.0 + 1.2e6 * r : 300000.0;
 }
 
-// The same as below for a lattice that may step with k_step4_flat (one list),
-// and whether it does.
+// The rule quads of a lattice that may step with k_step4_flat (one list), and
+// whether it does.
 // Leading blocks: `share` rule cells per thread for each wave of plain blocks:
 // channel 16 (256x128x127: 12 94.0, 24 82.3 us), walls alone 12 (8: 99.8, 16:
 // 88.9).
